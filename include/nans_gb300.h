@@ -134,9 +134,11 @@ typedef struct nans_contact_pair
                                       GJK, EPA on the per-thread and warp tiers, solve; a block
                                       per scene) after the sweep, in place of the staged
                                       kernels; EPAs beyond the warp tier still take the large
-                                      tiers and the late solve pass. Same results. For worlds of
-                                      small scenes, where the staged step's launch chain is the
-                                      cost (the reference's own scene). Scenes of at most 1,024
+                                      tiers and the late solve pass. Same results. For worlds of a
+                                      few small scenes, where the staged step's launch chain is
+                                      the cost (the reference's own scene); a world with a scene of
+                                      more than 24 bodies or more scenes than the GPU has SMs takes
+                                      the staged kernels, which are faster there. Scenes of at most 1,024
                                       bodies; the candidate buffers hold every pair (the
                                       max_candidates request is raised to that); not with
                                       NANS_WORLD_WARM_START. nans_profile_steps and

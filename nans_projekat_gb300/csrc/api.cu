@@ -61,7 +61,7 @@ struct nans_world
     uint32_t max_cand_req = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;   // the later EPA tiers, alongside the first solve pass
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_pairs = nullptr;
     int sm_count = 0;
 
     int n_scenes = 0, n_dyn = 0, n_all = 0, n_cubes = 0, n_spheres = 0;
@@ -90,6 +90,8 @@ struct nans_world
     long long steps_run = 0;
 
     int narrow_bpsm = 0;     // GJK blocks per SM (0 = occupancy limit)
+    bool long_gjk = false;   // the long GJK runs take a thread each, not a warp
+    bool pair_only = false; // so few pairs that the narrowphase is the pair tier's launch alone
     int cull_tiles = 1;      // cull by tiles (1) or one lane per pair (0)
     int gjk_cap_blocks = 1;  // GJK blocks the world's pairs can keep busy
     int solve_threads0 = 0;  // solver threads per scene, first pass (0 = by the largest scene)
@@ -117,6 +119,7 @@ struct nans_world
     // differentiable rollout: the tape lives in a chunked device arena reused across forwards
     bool tape_on = false;           // the solve records its adjoint data (s_fwd, s_maxw)
     bool fused = false;             // NANS_WORLD_FUSED_STEP: one detect-and-solve launch per step
+    bool fused_small = false;       // its scenes are few and small enough to step faster that way
     bool fused_conditional = true;  // its graphs put the large tiers in a conditional node
     bool tape_valid = false;        // the tape describes the rollout that led to the state
     float tape_dt = 0.0f;
@@ -319,6 +322,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     int cube_rank = 0, sphere_rank = 0, b = 0, max_bodies = 0;
     long long pair_acc = 0;
     long long hull_off = 0;
+    bool large_hulls = false; // a hull of more than eight points
     for (int s = 0; s < S; ++s)
     {
         sc_cube0[s] = b;
@@ -350,6 +354,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
             if (np > 0)
             {
                 sh.y = np;
+                large_hulls = large_hulls || np > 8;
                 sh.z = (int)local.size();
                 for (int k = 0; k < 3 * np; ++k)
                     local.push_back(hull_pts[3 * hull_off + k]);
@@ -517,6 +522,20 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     w->medium_cap_blocks = upto(4, INT32_MAX);
     d.medium_blocks = std::min(w->medium_bpsm * w->sm_count, w->medium_cap_blocks);
     d.tiny_blocks = upto(64, epa_tiny_grid(w->sm_count));
+    d.pair_blocks = upto(2, pair_warp_grid(w->sm_count));
+    // The fused step runs a scene on one block, so it pays while a scene's pairs fit the block's warps
+    // and every scene has an SM: 57.7 against 73.6 us a step for one scene of 9 bodies and 58.0 against
+    // 69.4 for 16, but 103 against 90 for 32 and 377 against 114 for 256.
+    w->fused_small = w->fused && max_bodies <= kSceneStepBodies && S <= w->sm_count;
+    // Steps of up to 16 candidates per SM give each pair a warp from the start of its GJK (136 against
+    // 142 us a step at 2,000 candidates; 197 against 162 at 6,400: then a thread per pair).
+    d.pair_max = 16 * w->sm_count;
+    w->pair_only = pair_acc <= d.pair_max && !(w->flags & NANS_WORLD_GJK_WARP);
+    // The long GJK runs (~1.5 % of the candidates) take a thread each in worlds of many boxes and
+    // spheres, where a warp each costs more issue slots than the shorter chain saves: 0.371 against
+    // 0.410 ms a step at 122,000 bodies, 0.223 against 0.208 at 34,000. Hulls of many points always
+    // take a warp (0.351 against 0.522 ms at 53,000 bodies).
+    w->long_gjk = ndyn >= 80000 && !large_hulls;
     d.gjk_warp = (w->flags & NANS_WORLD_GJK_WARP) ? 1 : 0;
     d.sm_count = w->sm_count;
     d.giant_blocks = std::min(giant_grid(w->sm_count), upto(1, INT32_MAX) < 4096 ? 16 : INT32_MAX);
@@ -642,6 +661,40 @@ void enqueue_cull(nans_world *w)
         k_cull_write<<<w->cull_blocks, kCullThreads, 0, st>>>(w->dw);
 }
 
+// GJK and the EPA tiers of every pair that does not outgrow the pair tier, on the world's stream;
+// with `beside`, what the GJK pass leaves to the pair tier (a few pairs, each a long chain of
+// dependent iterations) runs on the second stream beside the per-thread EPA. A world of few pairs
+// runs the pair tier alone: two launches fewer, and no pair waits for the lanes of 31 others.
+cudaError_t enqueue_narrow(nans_world *w, bool beside)
+{
+    cudaStream_t st = w->stream, st2 = beside ? w->stream2 : w->stream;
+    if (w->pair_only)
+    {
+        launch_pair_warp(st, w->dw, PAIRS_ALL);
+        return cudaGetLastError();
+    }
+    cudaError_t e = cudaSuccess;
+    launch_gjk(narrow_grid(w), st, w->dw);
+    if (beside)
+    {
+        e = cudaEventRecord(w->ev_fork, st);
+        if (e == cudaSuccess)
+            e = cudaStreamWaitEvent(st2, w->ev_fork, 0);
+        if (e != cudaSuccess)
+            return e;
+    }
+    if (w->long_gjk)
+        launch_gjk_long(narrow_grid(w), st2, w->dw);
+    launch_pair_warp(st2, w->dw, PAIRS_FRONT);
+    if (beside)
+        e = cudaEventRecord(w->ev_pairs, st2);
+    launch_epa_tiny(st, w->dw);
+    launch_pair_warp(st, w->dw, PAIRS_BACK);
+    if (beside && e == cudaSuccess)
+        e = cudaStreamWaitEvent(st, w->ev_pairs, 0);
+    return e;
+}
+
 // Narrowphase and solve. The EPA tiers beyond the per-thread one run on the second stream
 // while the first solve pass handles every scene they do not touch; the second pass solves
 // the rest after them. Both streams are joined before the function returns (also under
@@ -651,10 +704,12 @@ void enqueue_cull(nans_world *w)
 cudaError_t enqueue_narrow_solve(nans_world *w, float dt, cudaEvent_t *tl)
 {
     cudaStream_t st = w->stream, st2 = w->stream2;
-    launch_narrow_tiny(narrow_grid(w), st, w->dw);
+    cudaError_t e = enqueue_narrow(w, true);
+    if (e != cudaSuccess)
+        return e;
     if (tl)
         cudaEventRecord(tl[0], st);
-    cudaError_t e = cudaEventRecord(w->ev_fork, st);
+    e = cudaEventRecord(w->ev_fork, st);
     if (e == cudaSuccess)
         e = cudaStreamWaitEvent(st2, w->ev_fork, 0);
     if (e != cudaSuccess)
@@ -703,11 +758,12 @@ void after_step(nans_world *w, float dt)
     ++w->steps_run;
 }
 
-// The fused step (NANS_WORLD_FUSED_STEP, not while a tape is recorded): the sweep (which also
+// The fused step (NANS_WORLD_FUSED_STEP, worlds of few small scenes, not while a tape is recorded): the
+// sweep (which also
 // clears the work counters), one launch that culls, collides and solves every scene, then the
 // large EPA tiers and the late solve pass for the scenes with an EPA beyond the warp tier. The
 // candidate buffers hold every pair, so nothing is read back.
-bool use_fused(const nans_world *w) { return w->fused && !w->tape_on; }
+bool use_fused(const nans_world *w) { return w->fused_small && !w->tape_on; }
 
 // The large EPA tiers and the late solve pass on stream st.
 cudaError_t enqueue_fused_tail(nans_world *w, float dt, cudaStream_t st)
@@ -1284,6 +1340,8 @@ int nans_world_create(const nans_world_desc *desc, nans_world **out)
     if (e == cudaSuccess)
         e = cudaEventCreateWithFlags(&w->ev_join, cudaEventDisableTiming);
     if (e == cudaSuccess)
+        e = cudaEventCreateWithFlags(&w->ev_pairs, cudaEventDisableTiming);
+    if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&w->sm_count, cudaDevAttrMultiProcessorCount, w->device);
     if (e == cudaSuccess)
         e = (cudaError_t)narrow_kernel_attrs();
@@ -1299,6 +1357,8 @@ int nans_world_create(const nans_world_desc *desc, nans_world **out)
             cudaEventDestroy(w->ev_fork);
         if (w->ev_join)
             cudaEventDestroy(w->ev_join);
+        if (w->ev_pairs)
+            cudaEventDestroy(w->ev_pairs);
         delete w;
         return fail(NANS_ERR_CUDA, std::string("create: ") + cudaGetErrorString(e));
     }
@@ -1334,6 +1394,8 @@ int nans_world_destroy(nans_world *w)
         cudaEventDestroy(w->ev_fork);
     if (w->ev_join)
         cudaEventDestroy(w->ev_join);
+    if (w->ev_pairs)
+        cudaEventDestroy(w->ev_pairs);
     delete w;
     return NANS_OK;
 }
@@ -2025,7 +2087,7 @@ int nans_profile_steps(nans_world *w, float dt, uint32_t nsteps, float *stage_ms
         CK(cudaEventRecord(ev[1], st));
         enqueue_cull(w);
         CK(cudaEventRecord(ev[2], st));
-        launch_narrow_tiny(narrow_grid(w), st, w->dw);
+        CK(enqueue_narrow(w, false));
         CK(cudaEventRecord(ev[3], st));
         launch_epa_medium(st, w->dw);
         CK(cudaEventRecord(ev[4], st));
@@ -2110,10 +2172,12 @@ int nans_launches_per_step(nans_world *w, uint32_t *batched, uint32_t *plain)
 {
     if (!w)
         return fail(NANS_ERR_INVALID_ARGUMENT, "launches: null world");
-    // sweep, [cull mask, cull write], cull scan, gjk, gjk_long, epa_tiny, epa_medium, block
-    // EPA, giant EPA, solve (two passes); fused: sweep, scene step, block EPA, giant EPA, late
-    // solve
-    uint32_t k = w->fused ? 5u : 10 + (w->cull_blocks > 0 ? 2u : 0u);
+    // sweep, [cull mask, cull write], cull scan, the narrowphase (the pair tier alone, or GJK,
+    // [its long runs], the pair tier's front, the per-thread EPA, the pair tier's back), epa_medium,
+    // block EPA, giant EPA, solve (two passes); fused: sweep, scene step, block EPA, giant EPA,
+    // late solve
+    const uint32_t narrow = w->pair_only ? 1u : (w->long_gjk ? 5u : 4u);
+    uint32_t k = w->fused_small ? 5u : 7 + narrow + (w->cull_blocks > 0 ? 2u : 0u);
     if (batched)
         *batched = k;
     if (plain)

@@ -1,35 +1,40 @@
-// Narrowphase tiers 1 and 2: GJK per candidate pair (one lane each), then EPA per hit, one
-// per thread on a 12-vertex / 20-face polytope (tier 1) and, for the EPAs that outgrow it,
-// one per warp on a 256-face polytope (tier 2; tiers 3 and 4 are in k_epa_large.cu).
+// Narrowphase: GJK per candidate pair, then EPA per hit.
+//
+//   k_gjk        one thread per pair, up to kGjkShort EvolveSimplex calls
+//   k_epa_tiny   one thread per hit, an 11-vertex / 16-face polytope (98 % of the EPAs)
+//   k_pair_warp  one warp per pair (nans_epa_warp.cuh, a 34-vertex / 64-face polytope in
+//                registers): the GJK runs that need more calls, the EPAs of hulls of many points
+//                and those the per-thread polytope does not hold; every pair of a step that has
+//                too few of them for a thread each
+//   k_gjk_long   the long GJK runs with a thread each, where there are very many
+//   k_epa_medium one warp per EPA beyond that, a 256-face polytope in shared memory with the
+//                reference's list semantics in full (tiers 3 and 4 are in k_epa_large.cu)
+//   k_scene_step the fused per-scene step
 //
 // GJK follows CheckCollision / EvolveSimplex (code/nans.cpp:571-769, 906-966): the search
 // direction is reset to normalize(PB - PA) on every call, Simplex[0] is the oldest point,
 // at most 65 calls, the degenerate-direction exit at |d| <= 1e-4 and the support test
-// dot(d, P) >= 0. The simplex lives in registers as four named slots. k_gjk gives each pair
-// 8 calls; pairs still evolving are queued with their simplex and call index and resumed by
-// k_gjk_long, so that long runs share warps with each other. A hit's final simplex is stored
-// for the EPA. The tier-1 queue is ordered in two parts: pairs whose EPA ran more than a few
-// iterations at the previous step first, then the rest, so that a warp's lanes run EPAs of
-// similar length.
+// dot(d, P) >= 0. A hit's final simplex is stored for the EPA.
 //
 // EPA follows ResolveCollision (code/nans.cpp:217-328, 771-904) with the polytope in
-// fixed-capacity shared-memory buffers instead of std::vector:
+// fixed-capacity buffers instead of std::vector:
 //   * vertices are a pool (GJK tetrahedron + one support per iteration);
 //   * faces are an ordered list of vertex indices with their normal and distance; removing
-//     the visible faces is a stable compaction, new faces are appended in edge order -- the
+//     the visible faces keeps the others' order, new faces are appended in edge order -- the
 //     same order vector::erase / push_back produce;
 //   * horizon edges are pushed in the order of the visible faces, each push cancelling the
-//     FIRST stored edge that is its reverse (vertex equality compares P, code/nans.h:251-254);
-//     the warp tier decides every push's fate in parallel from its group of equal edges.
+//     FIRST stored edge that is its reverse (vertex equality compares P, code/nans.h:251-254).
 // A face's "recomputed" normal in the closest-face search and the removal test equals its
-// stored normal bit for bit (same operands, same operations, the flip is an exact negation),
-// so each face's distance |dot(N, A)| is computed once, when the face is created or kept.
+// stored normal bit for bit (same operands, same operations, the flip is an exact negation).
 // An EPA whose support point no face sees ends at once: nothing changes, so every later
-// iteration would repeat it up to the cap. Tier 1 runs one EPA per thread; tier 2 one per
-// warp, whose lanes share the per-face loops while the sequential parts run redundantly.
+// iteration would repeat it up to the cap.
+//
+// 16,384 stacks (0.95 M pairs a step): the per-thread EPA takes 275 us where the form with the
+// horizon inside the face loop and a 20-face polytope took 535, and 1 in 1,000 of the EPAs it sends
+// on goes beyond the pair tier (1 in 250 went to the 256-face tier before).
 #include <algorithm>
 
-#include "nans_gjk.cuh"
+#include "nans_epa_warp.cuh"
 #include "nans_solve.cuh"
 
 namespace nans
@@ -463,6 +468,8 @@ __device__ int epa_run(const DevWorld &w, B &E, const Shape &A, const Shape &Bs,
 }
 
 
+constexpr int kPairThreads = 64;
+
 // Returns the tier-3 queue index (the caller may leave its state in handover[q]), or -1.
 __device__ __forceinline__ int escalate(const DevWorld &w, int c, bool to_big)
 {
@@ -530,31 +537,25 @@ __device__ __forceinline__ void handover_put(const DevWorld &w, const EpaFast &E
 }
 
 // ------------------------------------------------------------------------------------
-// Tier 1: one thread per candidate pair, GJK then EPA on a small per-thread polytope.
-// Positions of the polytope's vertices, its faces and the horizon live in shared memory in
-// field-major layout ([slot][thread], so a warp touches 32 consecutive words); the support
-// points SupA/SupB, read only for the final contact point, live in thread-local arrays.
-// 12 vertices (8 EPA iterations) and 20 faces hold ~99.7% of the EPAs of the stack workload.
+// Tier 1: one thread per hit, EPA on a small per-thread polytope of distinct vertices. Vertex
+// positions and face normals live in shared memory in field-major layout ([slot][thread], so a
+// warp touches 32 consecutive words); the face list is an ordered list of slots in 4-bit steps of
+// one 64-bit word, so that removing faces moves nothing, and the horizon one byte per edge in
+// another. The support points SupA/SupB, read only for the final contact point, live in
+// thread-local arrays. 16 faces and 11 vertices (7 iterations) hold ~99% of the stack workload's
+// EPAs.
 // ------------------------------------------------------------------------------------
 constexpr int kTinyThreads = 64;
-#ifndef NANS_TINY_V
-#define NANS_TINY_V 12
-#endif
-#ifndef NANS_TINY_F
-#define NANS_TINY_F 20
-#endif
-constexpr int kTinyV = NANS_TINY_V;
-constexpr int kTinyF = NANS_TINY_F;
-constexpr int kTinyE = 12;
-constexpr unsigned kNoCanon = 15u; // a vertex with a NaN coordinate: equal to no vertex
-static_assert(kTinyV < 15, "vertex and canonical indices are packed in 4 bits");
+constexpr int kTinyV = 11;
+constexpr int kTinyF = 16;
+constexpr int kTinyE = 8;
+static_assert(kTinyV <= 15 && kTinyF <= 16 && kTinyE <= 8, "4-bit vertices and slots, one byte per edge");
 
 struct TinySmem
 {
     float px[kTinyV][kTinyThreads], py[kTinyV][kTinyThreads], pz[kTinyV][kTinyThreads];
     float fnx[kTinyF][kTinyThreads], fny[kTinyF][kTinyThreads], fnz[kTinyF][kTinyThreads];
-    unsigned fidx[kTinyF][kTinyThreads];       // a | b << 8 | c << 16
-    unsigned short edge[kTinyE][kTinyThreads]; // u | v << 4 | canon(u) << 8 | canon(v) << 12
+    unsigned short fidx[kTinyF][kTinyThreads]; // a | b << 4 | c << 8
 };
 
 struct TinyLocal
@@ -564,12 +565,15 @@ struct TinyLocal
 
 __device__ __forceinline__ v3 tiny_p(const TinySmem &S, int t, int i) { return mk3(S.px[i][t], S.py[i][t], S.pz[i][t]); }
 
-// Stores vertex i and returns its canonical index: the first vertex whose P equals it (P
-// equality is what the reference's edge matching compares), kNoCanon when P has a NaN.
-// `canon` holds the canonical indices of vertices 0..i-1, 4 bits each.
-__device__ __forceinline__ unsigned tiny_put(TinySmem &S, TinyLocal &L, int t, int i, const GV &g,
-                                             unsigned long long canon)
+// Stores vertex i. Returns false when its P has a NaN or equals an earlier vertex's: the
+// reference's edge matching compares positions (code/nans.h:251-254), and only with distinct
+// vertices does comparing their indices give the same.
+__device__ __forceinline__ bool tiny_put(TinySmem &S, TinyLocal &L, int t, int i, const GV &g)
 {
+    bool distinct = !(isnan(g.p.x) || isnan(g.p.y) || isnan(g.p.z));
+    for (int j = 0; j < i; ++j)
+        if (eq3(tiny_p(S, t, j), g.p))
+            distinct = false;
     S.px[i][t] = g.p.x;
     S.py[i][t] = g.p.y;
     S.pz[i][t] = g.p.z;
@@ -579,61 +583,49 @@ __device__ __forceinline__ unsigned tiny_put(TinySmem &S, TinyLocal &L, int t, i
     L.sb[i][0] = g.sb.x;
     L.sb[i][1] = g.sb.y;
     L.sb[i][2] = g.sb.z;
-    if (isnan(g.p.x) || isnan(g.p.y) || isnan(g.p.z))
-        return kNoCanon;
-    for (int j = 0; j < i; ++j)
-        if (eq3(tiny_p(S, t, j), g.p))
-            return (unsigned)(canon >> (4 * j)) & 15u;
-    return (unsigned)i;
+    return distinct;
 }
 
 // PushTriangle (code/nans.cpp:292-322); returns the face's distance |dot(N, A)|, which the
 // reference recomputes from the same operands in its closest-face search (bit-equal).
-__device__ __forceinline__ float tiny_face(TinySmem &S, int t, int f, int a, int b, int c)
+__device__ __forceinline__ float tiny_face(TinySmem &S, int t, int f, int a, int b, int c, v3 pa)
 {
-    v3 pa = tiny_p(S, t, a), pb = tiny_p(S, t, b), pc = tiny_p(S, t, c);
+    v3 pb = tiny_p(S, t, b), pc = tiny_p(S, t, c);
     v3 n = normalize3(cross3(pb - pa, pc - pa));
     if (dot3(pa, n) < 0.0f)
         n = -1.0f * n;
-    S.fidx[f][t] = (unsigned)a | ((unsigned)b << 8) | ((unsigned)c << 16);
+    S.fidx[f][t] = (unsigned short)(a | (b << 4) | (c << 8));
     S.fnx[f][t] = n.x;
     S.fny[f][t] = n.y;
     S.fnz[f][t] = n.z;
     return fabsf(dot3(n, pa));
 }
 
-// PushEdge (code/nans.cpp:232-266), sequential. The stored edge (x, y) is the reverse of (u, v)
-// when P(x) == P(v) and P(y) == P(u): equal canonical indices (a NaN vertex matches nothing).
-// Returns false on overflow.
-__device__ __forceinline__ bool tiny_edge(TinySmem &S, int t, unsigned long long canon, int &ne, int u, int v)
+// PushEdge (code/nans.cpp:232-266) on a list of up to eight edges (u | v << 4, one byte each, in
+// push order from the low byte): the first stored edge that is the reverse of (u, v) leaves, or
+// (u, v) is appended. No edge is 0 (u != v), so the bytes beyond the list match nothing. Returns
+// false when the list is full.
+__device__ __forceinline__ bool tiny_edge(unsigned long long &list, int &ne, unsigned u, unsigned v)
 {
-    const unsigned cu = (unsigned)(canon >> (4 * u)) & 15u, cv = (unsigned)(canon >> (4 * v)) & 15u;
-    if (cu != kNoCanon && cv != kNoCanon)
+    const unsigned pat = (v | (u << 4)) * 0x01010101u;
+    const unsigned xl = (unsigned)list ^ pat, xh = (unsigned)(list >> 32) ^ pat;
+    // the lowest zero byte's top bit
+    const unsigned zl = (xl - 0x01010101u) & ~xl & 0x80808080u, zh = (xh - 0x01010101u) & ~xh & 0x80808080u;
+    if (zl | zh)
     {
-        const unsigned want = cv | (cu << 4);
-        for (int e = 0; e < ne; ++e)
-        {
-            if ((unsigned)(S.edge[e][t] >> 8) == want)
-            {
-                for (int k = e + 1; k < ne; ++k)
-                    S.edge[k - 1][t] = S.edge[k][t];
-                --ne;
-                return true;
-            }
-        }
+        const int bit = zl ? __ffs(zl) - 8 : __ffs(zh) + 24;
+        const unsigned long long low = (1ull << bit) - 1ull;
+        list = (list & low) | ((list >> 8) & ~low);
+        --ne;
+        return true;
     }
     if (ne >= kTinyE)
         return false;
-    S.edge[ne][t] = (unsigned short)(u | (v << 4) | (cu << 8) | (cv << 12));
+    list |= (unsigned long long)(u | (v << 4)) << (8 * ne);
     ++ne;
     return true;
 }
 
-// ResolveCollision (code/nans.cpp:787-904) by one thread; same results as epa_run.
-// `simp` is the GJK simplex as the GJK pass stored it (4 x (P, SupA, SupB), 36 floats).
-// The closest-face search of the next iteration is folded into the removal pass and the face
-// creation: a running minimum with strict '<' over the kept faces, then the new ones, in list
-// order, is the reference's scan (a NaN first distance keeps face 0, as its scan does).
 // The 8 world vertices of an 8-point shape (a box) in registers: the per-thread EPA's support
 // maps read them once per EPA instead of at every iteration (the polytopes' shared memory leaves
 // the L1 little room). box_support is hull_support's scan: the same order, products and strict
@@ -681,6 +673,17 @@ __device__ __forceinline__ v3 box_support(const Verts8 &r, v3 d)
     return out;
 }
 
+// ResolveCollision (code/nans.cpp:787-904) by one thread; same results as epa_run and epa_warp,
+// or EPA_OVERFLOW for a polytope it does not hold: one that outgrows it, has a repeated or NaN
+// vertex, or loses every face.
+// `simp` is the GJK simplex as the GJK pass stored it (4 x (P, SupA, SupB), 36 floats).
+// Every running EPA of a warp is at the same iteration and a regular polytope has 4 + 2 it faces,
+// so the face loop is uniform; it only marks the visible faces, whose edges (one or two faces in
+// 97 % of the iterations) then follow in a loop of their own. With the edges inside the face loop
+// a warp ran them for nearly every face, for a few lanes each.
+// The closest-face search of the next iteration is folded into the face loop and the face
+// creation: a running minimum with strict '<' over the kept faces, then the new ones, in list
+// order, is the reference's scan (a NaN first distance keeps face 0, as its scan does).
 __device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, const Shape &B, const float *simp,
                         v3 &out_pa, v3 &out_pb, v3 &out_n, int &iters)
 {
@@ -691,7 +694,8 @@ __device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, c
         load_verts8(w.verts, A.off, VA);
     if (rb)
         load_verts8(w.verts, B.off, VB);
-    unsigned long long canon = 0ull;
+    bool distinct = true;
+#pragma unroll
     for (int i = 0; i < 4; ++i)
     {
         const float *q = simp + 9 * i;
@@ -699,38 +703,32 @@ __device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, c
         g.p = mk3(q[0], q[1], q[2]);
         g.sa = mk3(q[3], q[4], q[5]);
         g.sb = mk3(q[6], q[7], q[8]);
-        canon |= (unsigned long long)tiny_put(S, L, t, i, g, canon) << (4 * i);
+        distinct = tiny_put(S, L, t, i, g) && distinct;
     }
-    float cur = tiny_face(S, t, 0, 0, 1, 2);
-    int ci = 0;
+    if (!distinct)
+        return EPA_OVERFLOW;
+    float cur = 0.0f;
+    int cs = 0; // slot of the closest face
+#pragma unroll 1
+    for (int f = 0; f < 4; ++f)
     {
-        const float d1 = tiny_face(S, t, 1, 0, 2, 3);
-        if (d1 < cur)
+        // ABC, ACD, ADB, BDC (code/nans.cpp:799-802)
+        const int a = f == 3 ? 1 : 0, b = f == 0 ? 1 : (f == 1 ? 2 : 3), c = f == 0 ? 2 : (f == 1 ? 3 : (f == 2 ? 1 : 2));
+        const float d = tiny_face(S, t, f, a, b, c, tiny_p(S, t, a));
+        if (f == 0 || d < cur)
         {
-            cur = d1;
-            ci = 1;
-        }
-        const float d2 = tiny_face(S, t, 2, 0, 3, 1);
-        if (d2 < cur)
-        {
-            cur = d2;
-            ci = 2;
-        }
-        const float d3 = tiny_face(S, t, 3, 1, 3, 2);
-        if (d3 < cur)
-        {
-            cur = d3;
-            ci = 3;
+            cur = d;
+            cs = f;
         }
     }
+    unsigned long long order = 0x3210ull;
+    unsigned used = 0xfu;
     int nf = 4, nv = 4;
-    bool stale = false;
+#pragma unroll 1
     for (int it = 0; it <= 64; ++it)
     {
         iters = it + 1;
-        if (nf == 0 && !stale)
-            return EPA_NONE;
-        const v3 n = mk3(S.fnx[ci][t], S.fny[ci][t], S.fnz[ci][t]);
+        const v3 n = mk3(S.fnx[cs][t], S.fny[cs][t], S.fnz[cs][t]);
         GV ns;
         ns.sa = ra ? box_support(VA, n) : shape_support(w.verts, A, n);
         const v3 nd = -1.0f * n;
@@ -738,8 +736,8 @@ __device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, c
         ns.p = ns.sa - ns.sb;
         if (dot3(n, ns.p) - cur < 0.001f)
         {
-            unsigned fi = S.fidx[ci][t];
-            int ia = fi & 0xffu, ib = (fi >> 8) & 0xffu, ic = fi >> 16;
+            const unsigned fi = S.fidx[cs][t];
+            const int ia = fi & 15u, ib = (fi >> 4) & 15u, ic = fi >> 8;
             v3 pa = tiny_p(S, t, ia), pb = tiny_p(S, t, ib), pc = tiny_p(S, t, ic);
             v3 p = cur * n;
             v3 v0 = pb - pa, v1 = pc - pa, v2 = p - pa;
@@ -762,75 +760,77 @@ __device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, c
             out_pb = ((bu * sba) + (bv * sbb)) + (bw * sbc);
             return EPA_CONTACT;
         }
-        if (nf == 0)
-            return EPA_NONE; // the stale read repeats identically until the iteration cap
-        // visible faces -> horizon edges, the others compacted in place (code/nans.cpp:869-891),
-        // with the running closest-face search over the kept ones
-        int ne = 0, keep = 0, nci = 0;
+        // the faces in list order: visible ones marked, the others kept (code/nans.cpp:869-891)
+        unsigned vism = 0u;
+        unsigned long long kept = 0ull, o = order;
+        int keep = 0, ncs = -1;
         float ncur = 0.0f;
-        for (int f = 0; f < nf; ++f)
+#pragma unroll 2
+        for (int f = 0; f < nf; ++f, o >>= 4)
         {
-            unsigned fi = S.fidx[f][t];
-            v3 fa = tiny_p(S, t, fi & 0xffu);
-            v3 fn = mk3(S.fnx[f][t], S.fny[f][t], S.fnz[f][t]);
+            const int slot = (int)o & 15;
+            const v3 fa = tiny_p(S, t, S.fidx[slot][t] & 15u);
+            const v3 fn = mk3(S.fnx[slot][t], S.fny[slot][t], S.fnz[slot][t]);
+            const float d = fabsf(dot3(fn, fa));
             if (dot3(fn, ns.p - fa) > 0.0f)
-            {
-                int a = fi & 0xffu, b = (fi >> 8) & 0xffu, c = fi >> 16;
-                if (!(tiny_edge(S, t, canon, ne, a, b) && tiny_edge(S, t, canon, ne, b, c) &&
-                      tiny_edge(S, t, canon, ne, c, a)))
-                    return EPA_OVERFLOW;
-            }
+                vism |= 1u << slot;
             else
             {
-                if (keep != f)
-                {
-                    S.fidx[keep][t] = fi;
-                    S.fnx[keep][t] = fn.x;
-                    S.fny[keep][t] = fn.y;
-                    S.fnz[keep][t] = fn.z;
-                }
-                const float d = fabsf(dot3(fn, fa));
+                kept |= (unsigned long long)slot << (4 * keep);
                 if (keep == 0 || d < ncur)
                 {
                     ncur = d;
-                    nci = keep;
+                    ncs = slot;
                 }
                 ++keep;
             }
         }
-        if (keep == nf)
+        if (vism == 0u)
             return EPA_NONE; // no face sees the support: every later iteration repeats this one
-        if (keep + ne > kTinyF || nv >= kTinyV)
-            return EPA_OVERFLOW;
-        if (keep == 0 && ne == 0)
+        // the visible faces' edges, in list order
+        unsigned long long edges = 0ull;
+        int ne = 0;
+        bool fits = nv < kTinyV;
+        o = order;
+        for (int left = nf - keep; left > 0; --left)
         {
-            // every face removed: slot 0 keeps the last face of the list (nothing was moved)
-            int l = nf - 1;
-            const unsigned fi = S.fidx[l][t];
-            const v3 fn = mk3(S.fnx[l][t], S.fny[l][t], S.fnz[l][t]);
-            S.fidx[0][t] = fi;
-            S.fnx[0][t] = fn.x;
-            S.fny[0][t] = fn.y;
-            S.fnz[0][t] = fn.z;
-            ncur = fabsf(dot3(fn, tiny_p(S, t, fi & 0xffu)));
-            nci = 0;
-            stale = true;
+            while (!((vism >> ((int)o & 15)) & 1u))
+                o >>= 4;
+            const unsigned fi = S.fidx[(int)o & 15][t];
+            o >>= 4;
+            const unsigned a = fi & 15u, b = (fi >> 4) & 15u, c = fi >> 8;
+            if (ne == 0)
+            {
+                // nothing to cancel: a face's own edges are no reverses of each other
+                edges = (a | (b << 4)) | ((b | (c << 4)) << 8) | ((c | (a << 4)) << 16);
+                ne = 3;
+            }
+            else
+                fits = tiny_edge(edges, ne, a, b) && tiny_edge(edges, ne, b, c) && tiny_edge(edges, ne, c, a) && fits;
         }
-        int sv = nv++;
-        canon |= (unsigned long long)tiny_put(S, L, t, sv, ns, canon) << (4 * sv);
-        for (int j = 0; j < ne; ++j)
+        if (!fits || keep + ne > kTinyF || keep + ne == 0)
+            return EPA_OVERFLOW;
+        used &= ~vism;
+        const int sv = nv++;
+        if (!tiny_put(S, L, t, sv, ns))
+            return EPA_OVERFLOW;
+        order = kept;
+        nf = keep;
+        for (int j = 0; j < ne; ++j, edges >>= 8)
         {
-            const unsigned ed = S.edge[j][t];
-            const float d = tiny_face(S, t, keep + j, sv, ed & 15u, (ed >> 4) & 15u);
-            if (keep + j == 0 || d < ncur)
+            const int slot = __ffs(~used) - 1;
+            used |= 1u << slot;
+            order |= (unsigned long long)slot << (4 * nf);
+            const float d = tiny_face(S, t, slot, sv, (int)edges & 15, ((int)edges >> 4) & 15, ns.p);
+            if (nf == 0 || d < ncur)
             {
                 ncur = d;
-                nci = keep + j;
+                ncs = slot;
             }
+            ++nf;
         }
-        nf = keep + ne;
         cur = ncur;
-        ci = nci;
+        cs = ncs;
     }
     return EPA_NONE;
 }
@@ -855,15 +855,46 @@ __device__ __forceinline__ void store_simplex(const DevWorld &w, int c, const GV
     o[8] = make_float4(s3.sa.z, s3.sb.x, s3.sb.y, s3.sb.z);
 }
 
-// Appends c to the EPA queue when `hit` (one atomic per warp and part). Pairs whose EPA took
-// more than kEpaLongIters iterations at its last step fill the queue from the back (count in
-// work counter 9), the others from the front (work counter 10): the per-thread EPA pass takes
-// the long ones first, so that the lanes of a warp run EPAs of similar length.
-constexpr int kEpaLongIters = 4;
-__device__ __forceinline__ void enqueue_epa(const DevWorld &w, int c, bool hit)
+// The pair tier's queue entries (long_cand): candidate and state. An unfinished GJK run is
+// n | it << 8 (n points, `it` calls made; 0 for a run not begun), an EPA to run from the stored
+// simplex kPairEpa. What the GJK pass queues fills the front (work counter 7) and runs beside the
+// per-thread EPA; what that leaves over fills the back (work counter 4) and runs after it. A
+// candidate is queued at most once, so the two never meet.
+constexpr int kPairEpa = 1 << 16;
+
+// Appends candidate c with `state` to a part of the pair tier's queue when `take`; one atomic
+// per warp.
+__device__ __forceinline__ void enqueue_pair(const DevWorld &w, int c, int state, bool back, bool take)
 {
     const unsigned act = __activemask();
-    const bool lng = hit && w.epa_hist[w.cand_pidx[c]] > kEpaLongIters;
+    const unsigned bal = __ballot_sync(act, take);
+    if (!take)
+        return;
+    const int lane = threadIdx.x & 31, leader = __ffs(bal) - 1;
+    int base = 0;
+    if (lane == leader)
+        base = atomicAdd(w.work_counter + (back ? 4 : 7), __popc(bal));
+    base = __shfl_sync(bal, base, leader);
+    const int k = base + __popc(bal & ((1u << lane) - 1u));
+    if (dev_check(w, k < w.cand_cap, 14, k, w.cand_cap))
+        w.long_cand[back ? w.cand_cap - 1 - k : k] = make_int2(c, state);
+}
+
+// Appends c to the per-thread EPA queue when `hit` (one atomic per warp and part). Pairs whose EPA
+// took more than kEpaLongIters iterations at its last step fill the queue from the back (count in
+// work counter 9), the others from the front (work counter 10): the per-thread EPA pass takes
+// the long ones first, so that the lanes of a warp run EPAs of similar length. Pairs whose last
+// EPA would not have fitted the per-thread polytope go to the pair tier at once.
+constexpr int kEpaLongIters = 4;
+constexpr int kEpaTinyIters = kTinyV - 3; // iterations a regular EPA can have on the per-thread polytope
+__device__ __forceinline__ void enqueue_epa(const DevWorld &w, int c, bool hit, bool hull)
+{
+    const int last = hit ? w.epa_hist[w.cand_pidx[c]] : 0;
+    const bool pair = hit && (hull || last > kEpaTinyIters);
+    enqueue_pair(w, c, kPairEpa, false, pair);
+    const unsigned act = __activemask();
+    hit = hit && !pair;
+    const bool lng = hit && last > kEpaLongIters;
     const unsigned bal = __ballot_sync(act, hit && !lng), ball = __ballot_sync(act, lng);
     if (!hit)
         return;
@@ -878,9 +909,6 @@ __device__ __forceinline__ void enqueue_epa(const DevWorld &w, int c, bool hit)
     w.s_order[lng ? w.cand_cap - 1 - k : k] = c;
 }
 
-// GJK of candidate c from call `it` with the simplex (s0..s3, n points). With a budget below
-// 65, a GJK still evolving is queued for the long pass with its state (the simplex in the
-// candidate's s_k slot, n and it in the queue), which resumes it.
 // Minkowski support with 8-point shapes' vertices in registers (Verts8), the others read from
 // memory: minkowski_support's values.
 struct RegSupport
@@ -900,8 +928,11 @@ struct RegSupport
     }
 };
 
-__device__ __forceinline__ void gjk_one(const DevWorld &w, int c, int ia, int ib, int budget, GV &s0, GV &s1, GV &s2,
-                                        GV &s3, int n, int it)
+// GJK of candidate c from call `it` with the simplex (s0..s3, n points), for up to `budget` calls. The
+// simplex of a hit and of a run still evolving goes to the candidate's slot; `hull` tells of a shape
+// of more than eight points.
+__device__ __forceinline__ int gjk_run(const DevWorld &w, int c, int ia, int ib, int budget, GV &s0, GV &s1, GV &s2,
+                                       GV &s3, int &n, int &it, bool &hull)
 {
     const Shape A = load_shape(w, ia), B = load_shape(w, ib);
     const bool ra = A.npts == 8, rb = B.npts == 8;
@@ -910,14 +941,11 @@ __device__ __forceinline__ void gjk_one(const DevWorld &w, int c, int ia, int ib
         load_verts8(w.verts, A.off, VA);
     if (rb)
         load_verts8(w.verts, B.off, VB);
+    hull = max(A.npts, B.npts) > 8;
     const int g = gjk_from_with(RegSupport{w.verts, A, B, ra, rb, VA, VB}, A, B, s0, s1, s2, s3, n, it, budget);
     if (g == G_FOUND || g == G_BUDGET)
         store_simplex(w, c, s0, s1, s2, s3);
-    if (g == G_BUDGET)
-        w.long_cand[atomicAdd(w.work_counter + 7, 1)] = make_int2(c, n | (it << 8));
-    else if (g != G_FOUND)
-        w.hit[c] = 0;
-    enqueue_epa(w, c, g == G_FOUND);
+    return g;
 }
 
 // Persistent: warps take 32 candidates at a time from a global queue; each lane runs GJK
@@ -963,7 +991,18 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
             if (c == n - 1 || (w.cand_meta[c + 1] >> 3) != sc)
                 w.cand_end[sc] = c + 1;
             GV s0 = {}, s1 = {}, s2 = {}, s3 = {};
-            gjk_one(w, c, ia, ib, kGjkShort, s0, s1, s2, s3, 0, 0);
+            if (n <= w.pair_max)
+                enqueue_pair(w, c, 0, false, true);
+            else
+            {
+                int np = 0, it = 0;
+                bool hull;
+                const int g = gjk_run(w, c, ia, ib, kGjkShort, s0, s1, s2, s3, np, it, hull);
+                if (g == G_NOHIT)
+                    w.hit[c] = 0;
+                enqueue_pair(w, c, np | (it << 8), false, g == G_BUDGET);
+                enqueue_epa(w, c, g == G_FOUND, hull);
+            }
         }
         base = next;
         ia = na;
@@ -971,14 +1010,17 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
     }
 }
 
-// The long pass: candidates whose GJK needed more than kGjkShort calls, resumed where the
-// first pass stopped.
+// The rest of the GJK runs that need more than kGjkShort calls, one thread each, for worlds with so
+// many of them that a warp each would cost more than the chain it shortens. The queue's entries
+// become EPAs (hits) or nothing (-1).
 __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk_long(DevWorld w)
 {
-    const int n = w.work_counter[7];
+    const int n = min(w.work_counter[7], w.cand_cap);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     {
         const int2 q = w.long_cand[i];
+        if (q.y == kPairEpa || !dev_check(w, q.x >= 0 && q.x < w.cand_cap, 16, q.x, w.cand_cap))
+            continue;
         const float4 *o = w.s_k + 9 * (size_t)q.x;
         const float4 k0 = o[0], k1 = o[1], k2 = o[2], k3 = o[3], k4 = o[4], k5 = o[5], k6 = o[6], k7 = o[7], k8 = o[8];
         GV s0, s1, s2, s3;
@@ -994,7 +1036,12 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk_long(DevWorld w)
         s3.p = mk3(k6.w, k7.x, k7.y);
         s3.sa = mk3(k7.z, k7.w, k8.x);
         s3.sb = mk3(k8.y, k8.z, k8.w);
-        gjk_one(w, q.x, w.cand_a[q.x], w.cand_b[q.x], 65, s0, s1, s2, s3, q.y & 0xff, q.y >> 8);
+        int np = q.y & 0xff, it = q.y >> 8;
+        bool hull;
+        const bool hit = gjk_run(w, q.x, w.cand_a[q.x], w.cand_b[q.x], 65, s0, s1, s2, s3, np, it, hull) == G_FOUND;
+        if (!hit)
+            w.hit[q.x] = 0;
+        w.long_cand[i] = make_int2(hit ? q.x : -1, kPairEpa);
     }
 }
 
@@ -1107,9 +1154,15 @@ __global__ void __launch_bounds__(kGjkWarpThreads) k_gjk_warp(DevWorld w)
             if (g == G_FOUND)
             {
                 store_simplex(w, c, s0, s1, s2, s3);
-                const bool lng = w.epa_hist[w.cand_pidx[c]] > kEpaLongIters;
-                const int k = atomicAdd(w.work_counter + (lng ? 9 : 10), 1);
-                w.s_order[lng ? w.cand_cap - 1 - k : k] = c;
+                const int last = w.epa_hist[w.cand_pidx[c]];
+                if (last > kEpaTinyIters || max(A.npts, B.npts) > 8)
+                    w.long_cand[atomicAdd(w.work_counter + 7, 1)] = make_int2(c, kPairEpa);
+                else
+                {
+                    const bool lng = last > kEpaLongIters;
+                    const int k = atomicAdd(w.work_counter + (lng ? 9 : 10), 1);
+                    w.s_order[lng ? w.cand_cap - 1 - k : k] = c;
+                }
             }
             else
                 w.hit[c] = 0;
@@ -1117,9 +1170,9 @@ __global__ void __launch_bounds__(kGjkWarpThreads) k_gjk_warp(DevWorld w)
     }
 }
 
-// Tier 1 EPA: one thread per hit from the queue; EPAs that outgrow the per-thread polytope
-// are queued for the warp tier.
-__global__ void __launch_bounds__(kTinyThreads) k_epa_tiny(DevWorld w)
+// Tier 1 EPA: one thread per hit from the queue; the polytopes it does not hold go to the pair
+// tier.
+__global__ void __launch_bounds__(kTinyThreads, 8) k_epa_tiny(DevWorld w)
 {
     __shared__ TinySmem S;
     const int lane = threadIdx.x & 31, t = threadIdx.x;
@@ -1146,13 +1199,84 @@ __global__ void __launch_bounds__(kTinyThreads) k_epa_tiny(DevWorld w)
         int iters = 0;
         const int r =
             epa_tiny(w, S, t, A, B, reinterpret_cast<const float *>(w.s_k + 9 * (size_t)c), pa, pb, nn, iters);
+        if (r != EPA_OVERFLOW)
+        {
+            const int pidx = w.cand_pidx[c];
+            if (dev_check(w, pidx >= 0 && pidx < w.n_words * 32, 11, pidx, (long long)w.n_words * 32))
+                w.epa_hist[pidx] = (unsigned char)iters;
+            write_result(w, c, r, pa, pb, nn);
+        }
+        enqueue_pair(w, c, kPairEpa, true, r == EPA_OVERFLOW);
+    }
+}
+
+// One pair by the whole warp (candidate c): the rest of its GJK when `gjk` is set (n points stored,
+// `it` calls made), then its EPA. Writes the candidate's hit and contact. Returns EPA_OVERFLOW for an
+// EPA that outgrew the warp's registers, its simplex in the candidate's slot.
+__device__ __forceinline__ int pair_warp(const DevWorld &w, WarpEpa &S, int c, bool gjk, int n, int it, int lane)
+{
+    const Shape A = load_shape(w, w.cand_a[c]), B = load_shape(w, w.cand_b[c]);
+    float *sq = reinterpret_cast<float *>(w.s_k + 9 * (size_t)c); // 36 floats, vertex by vertex
+    const v3 va = lane_vertex(w.verts, A, lane), vb = lane_vertex(w.verts, B, lane);
+    for (int k = lane; k < 9 * n; k += 32)
+        S.v[k % 9][k / 9] = sq[k];
+    __syncwarp();
+    if (gjk)
+    {
+        if (gjk_warp(w, S, A, B, va, vb, n, it, lane) != G_FOUND)
+        {
+            if (lane == 0)
+                w.hit[c] = 0;
+            return EPA_NONE;
+        }
+        for (int k = lane; k < 36; k += 32)
+            sq[k] = S.v[k % 9][k / 9]; // for the later tiers
+    }
+    v3 pa, pb, nn;
+    int iters = 0;
+    const int r = epa_warp(w, S, A, B, va, vb, lane, pa, pb, nn, iters);
+    if (lane == 0)
+    {
         const int pidx = w.cand_pidx[c];
         if (dev_check(w, pidx >= 0 && pidx < w.n_words * 32, 11, pidx, (long long)w.n_words * 32))
             w.epa_hist[pidx] = (unsigned char)(r == EPA_OVERFLOW ? 255 : iters);
-        if (r == EPA_OVERFLOW)
-            escalate(w, c, false);
-        else
+        if (r != EPA_OVERFLOW)
             write_result(w, c, r, pa, pb, nn);
+    }
+    __syncwarp();
+    return r;
+}
+
+// The pair tier: a warp per queued pair first finishes its GJK where the first pass left it (hulls
+// of more than eight points, runs of more than kGjkShort calls), then runs its EPA. EPAs that
+// outgrow the warp's registers are queued for the warp tier. Warps stride over the queue. `part`
+// names the entries: the queue's front or back, or every candidate from the start of its GJK.
+__global__ void __launch_bounds__(kPairThreads, 10) k_pair_warp(DevWorld w, int part)
+{
+    __shared__ WarpEpa sm[kPairThreads / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n = part == PAIRS_ALL ? *w.n_cand : min(w.work_counter[part == PAIRS_BACK ? 4 : 7], w.cand_cap);
+    // consecutive entries go to different blocks
+    for (int i = wid * gridDim.x + blockIdx.x; i < n; i += gridDim.x * (kPairThreads / 32))
+    {
+        int2 q = make_int2(i, 0);
+        if (part == PAIRS_ALL)
+        {
+            const int sc = w.cand_meta[i] >> 3;
+            if (lane == 0 && (i == 0 || (w.cand_meta[i - 1] >> 3) != sc))
+                w.cand_begin[sc] = i;
+            if (lane == 0 && (i == n - 1 || (w.cand_meta[i + 1] >> 3) != sc))
+                w.cand_end[sc] = i + 1;
+        }
+        else
+            q = w.long_cand[part == PAIRS_BACK ? w.cand_cap - 1 - i : i];
+        if (q.x == -1 || !dev_check(w, q.x >= 0 && q.x < w.cand_cap, 13, q.x, w.cand_cap))
+            continue;
+        const bool gjk = q.y != kPairEpa;
+        const int r = pair_warp(w, sm[wid], q.x, gjk, gjk ? q.y & 0xff : 4, q.y >> 8, lane);
+        if (r == EPA_OVERFLOW && lane == 0)
+            escalate(w, q.x, false);
+        __syncwarp();
     }
 }
 
@@ -1213,10 +1337,9 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32) k_epa_medium(
 //       when their inflated boxes meet (k_cull_mask's test), compacted in order by block scans
 //       into the scene's own slots of the pair space (from sc_word0 * 32: the candidate
 //       buffers of such a world hold every pair, so no scan across scenes is needed);
-//   (2) GJK, one thread per candidate, every EvolveSimplex call in one run;
-//   (3) EPA per hit on the per-thread polytope (epa_tiny);
-//   (4) the EPAs that outgrew it, one per warp on the warp tier's polytope (epa_run);
-//   (5) the solve (solve_scene), unless an EPA outgrew the warp tier: that pair goes to the
+//   (2) GJK and EPA, a warp per candidate (pair_warp);
+//   (3) the EPAs that outgrew its registers, one per warp on the warp tier's polytope (epa_run);
+//   (4) the solve (solve_scene), unless an EPA outgrew the warp tier: that pair goes to the
 //       block- and grid-wide tiers as in the staged step and its scene to the late solve pass.
 //       In a CUDA graph those launches sit in a conditional node, which the launch's last block
 //       to finish opens only when a scene went late.
@@ -1224,35 +1347,37 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32) k_epa_medium(
 // Every value the phases read from global memory was written by an earlier launch (the sweep)
 // or by the same block before a barrier.
 // ---------------------------------------------------------------------------------------
-constexpr int kSceneThreads = kTinyThreads; // the per-thread polytopes' shared-memory layout
+constexpr int kSceneThreads = 256;
+constexpr int kSceneWarpEpas = 2; // warps of the block that run warp-tier EPAs (shared memory)
 static_assert(kSceneThreads % 32 == 0 && kSceneThreads <= kWaveChunk, "scene step block size");
 // the block's dynamic shared memory stays within the 48 KB a launch gets without an opt-in
-static_assert(sizeof(TinySmem) <= 48 * 1024 && (kSceneThreads / 32) * sizeof(EpaFast) <= 48 * 1024 &&
+static_assert((kSceneThreads / 32) * sizeof(WarpEpa) <= 48 * 1024 &&
+                  kSceneWarpEpas * sizeof(EpaFast) <= 48 * 1024 &&
                   (size_t)(kSceneStepMaxBodies + 1) * 2 * sizeof(float4) <= 48 * 1024 &&
                   4 * kWaveChunk * sizeof(int) + kSceneStepMaxBodies * sizeof(int) <= 48 * 1024,
               "scene step shared memory");
 
 size_t scene_step_smem(size_t solve_bytes)
 {
-    return std::max(std::max(sizeof(TinySmem), (size_t)(kSceneThreads / 32) * sizeof(EpaFast)), solve_bytes);
+    return std::max(std::max((size_t)(kSceneThreads / 32) * sizeof(WarpEpa),
+                             (size_t)kSceneWarpEpas * sizeof(EpaFast)),
+                    solve_bytes);
 }
 
 __global__ void __launch_bounds__(kSceneThreads) k_scene_step(DevWorld w, float dt, int all_pairs,
                                                                cudaGraphConditionalHandle cond, int signal)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    TinySmem &S = *reinterpret_cast<TinySmem *>(smem_raw);
     EpaFast *const epa = reinterpret_cast<EpaFast *>(smem_raw);
     float4 *const s_dyn = reinterpret_cast<float4 *>(smem_raw);
     __shared__ int sh[32];
-    __shared__ int s_q, s_nq, s_nw, s_late, s_maxw;
+    __shared__ int s_q, s_nw, s_late, s_maxw;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (;;)
     {
         if (tid == 0)
         {
             s_q = atomicAdd(w.work_counter + 14, 1);
-            s_nq = 0;
             s_nw = 0;
             s_late = 0;
         }
@@ -1320,54 +1445,23 @@ __global__ void __launch_bounds__(kSceneThreads) k_scene_step(DevWorld w, float 
             w.scene_late[s] = 0;
         }
         __syncthreads(); // the last chunk's candidates, written after its scan
-        // (2) GJK; the hits' simplices go to their s_k slots and the hits to s_order[cb ..)
-        for (int c = cb + tid; c < ce; c += kSceneThreads)
+        // (2) GJK and EPA, a warp per candidate; the EPAs that outgrow its registers go to
+        // s_wave[cb ..)
+        for (int c = cb + wid; c < ce; c += kSceneThreads / 32)
         {
-            const Shape A = load_shape(w, w.cand_a[c]), B = load_shape(w, w.cand_b[c]);
-            const bool ra = A.npts == 8, rb = B.npts == 8;
-            Verts8 VA, VB;
-            if (ra)
-                load_verts8(w.verts, A.off, VA);
-            if (rb)
-                load_verts8(w.verts, B.off, VB);
-            GV s0 = {}, s1 = {}, s2 = {}, s3 = {};
-            int n = 0, it = 0;
-            const int g = gjk_from_with(RegSupport{w.verts, A, B, ra, rb, VA, VB}, A, B, s0, s1, s2, s3, n, it, 65);
-            if (g == G_FOUND)
-            {
-                store_simplex(w, c, s0, s1, s2, s3);
-                w.s_order[cb + atomicAdd(&s_nq, 1)] = c;
-            }
-            else
-                w.hit[c] = 0;
-        }
-        __syncthreads();
-        // (3) per-thread EPA; the EPAs that outgrow its polytope go to s_wave[cb ..)
-        const int nq = s_nq;
-        for (int i = tid; i < nq; i += kSceneThreads)
-        {
-            const int c = w.s_order[cb + i];
-            if (!dev_check(w, c >= cb && c < ce, 21, c, ce))
-                continue;
-            const Shape A = load_shape(w, w.cand_a[c]), B = load_shape(w, w.cand_b[c]);
-            v3 pa, pb, nn;
-            int iters = 0;
-            const int r =
-                epa_tiny(w, S, tid, A, B, reinterpret_cast<const float *>(w.s_k + 9 * (size_t)c), pa, pb, nn, iters);
-            w.epa_hist[w.cand_pidx[c]] = (unsigned char)(r == EPA_OVERFLOW ? 255 : iters);
-            if (r == EPA_OVERFLOW)
+            const int r = pair_warp(w, reinterpret_cast<WarpEpa *>(smem_raw)[wid], c, true, 0, 0, lane);
+            if (r == EPA_OVERFLOW && lane == 0)
             {
                 w.hit[c] = 0;
                 atomicAdd(w.epa_stats + 6, 1u);
                 w.s_wave[cb + atomicAdd(&s_nw, 1)] = c;
             }
-            else
-                write_result(w, c, r, pa, pb, nn);
+            __syncwarp();
         }
-        __syncthreads(); // the per-thread polytopes' memory becomes the warps' polytopes
-        // (4) warp tier, from the simplex the GJK phase stored
+        __syncthreads(); // the pairs' polytopes' memory becomes the warp tier's
+        // (3) warp tier, from the simplex the GJK stored
         const int nw = s_nw;
-        for (int i = wid; i < nw; i += kSceneThreads / 32)
+        for (int i = wid; i < nw && wid < kSceneWarpEpas; i += kSceneWarpEpas)
         {
             EpaFast &E = epa[wid];
             int cc = w.s_wave[cb + i];
@@ -1405,7 +1499,7 @@ __global__ void __launch_bounds__(kSceneThreads) k_scene_step(DevWorld w, float 
             __syncwarp();
         }
         __syncthreads(); // the warps' polytopes' memory becomes the solver's
-        // (5) the solve, unless a pair of the scene went to the large tiers (the late pass)
+        // (4) the solve, unless a pair of the scene went to the large tiers (the late pass)
         if (!s_late)
             solve_scene<false>(w, s, dt, s_dyn, sh, s_maxw);
         __syncthreads();
@@ -1465,16 +1559,11 @@ int epa_tiny_grid(int sm_count)
     return std::max(1, per) * std::max(1, sm_count);
 }
 
-void launch_narrow_tiny(int grid, cudaStream_t st, const DevWorld &w)
+int pair_warp_grid(int sm_count)
 {
-    if (w.gjk_warp)
-        k_gjk_warp<<<gjk_warp_grid(w), kGjkWarpThreads, 0, st>>>(w);
-    else
-    {
-        k_gjk<<<grid, kGjkThreads, 0, st>>>(w);
-        k_gjk_long<<<grid, kGjkThreads, 0, st>>>(w);
-    }
-    k_epa_tiny<<<w.tiny_blocks, kTinyThreads, 0, st>>>(w);
+    int per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_warp, kPairThreads, 0);
+    return std::max(1, per) * std::max(1, sm_count);
 }
 
 int tier_priority()
@@ -1487,6 +1576,34 @@ int tier_priority()
         prio = greatest;
     }
     return prio;
+}
+
+void launch_gjk(int grid, cudaStream_t st, const DevWorld &w)
+{
+    if (w.gjk_warp)
+        k_gjk_warp<<<gjk_warp_grid(w), kGjkWarpThreads, 0, st>>>(w);
+    else
+        k_gjk<<<grid, kGjkThreads, 0, st>>>(w);
+}
+
+void launch_gjk_long(int grid, cudaStream_t st, const DevWorld &w) { k_gjk_long<<<grid, kGjkThreads, 0, st>>>(w); }
+
+void launch_epa_tiny(cudaStream_t st, const DevWorld &w) { k_epa_tiny<<<w.tiny_blocks, kTinyThreads, 0, st>>>(w); }
+
+// The pair tier is launched at the greatest priority: beside the per-thread EPA its few long
+// chains must start first.
+void launch_pair_warp(cudaStream_t st, const DevWorld &w, int part)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(w.pair_blocks);
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributePriority;
+    attr[0].val.priority = tier_priority();
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_pair_warp, w, part);
 }
 
 // The escalation tiers are latency-bound chains on the step's critical path; they are

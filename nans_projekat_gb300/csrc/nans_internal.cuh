@@ -90,7 +90,8 @@ struct DevWorld
     float4 *c_pa, *c_pb, *c_n;
     int *work_counter;                  // [0] narrowphase head, [1] solver head, [2] block-EPA
                                         // head, [3] block-EPA queue length, [5] warp-EPA queue
-                                        // length, [6] warp-EPA head, [7] long-GJK queue length,
+                                        // length, [6] warp-EPA head, [7] pair-tier queue length
+                                        // (from the front) and [4] from the back,
                                         // [8] giant-EPA queue length, per-thread EPA queue
                                         // (s_order): [9] its long part (from the back), [10]
                                         // the others, [11] its head; [12] late-solve head,
@@ -98,9 +99,11 @@ struct DevWorld
                                         // head, [15] its blocks done
     int med_cap;                        // warp-EPA queue capacity
     int *med_cand;                      // candidates queued for the warp tier
-    int2 *long_cand;                    // candidates whose GJK needs the long pass: (c, n | it << 8)
+    int2 *long_cand;                    // the pair tier's queue: candidate and state
     int medium_blocks;                  // warp-tier grid
     int tiny_blocks;                    // per-thread EPA grid (resident blocks on every SM)
+    int pair_blocks;                   // pair-tier grid (resident blocks on every SM)
+    int pair_max;                      // steps of up to this many candidates run on the pair tier alone
     int gjk_warp;                       // 1: GJK with one warp per pair (NANS_WORLD_GJK_WARP)
     int sm_count;
     int ovf_cap;                        // block-EPA queue capacity

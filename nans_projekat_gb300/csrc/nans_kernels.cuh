@@ -37,7 +37,8 @@ constexpr int kSolveLateBlocksPerSm = 6; // second-pass solver blocks per SM (re
 constexpr int kWaveChunk = 256;     // solver: candidates compacted and labelled per chunk
 constexpr size_t kSolveSmemMax = 200 * 1024; // solver: dynamic shared memory per block, at most
 constexpr int kMediumBlocksPerSm = 2;    // warp-tier EPA blocks per SM (shared memory allows three)
-constexpr int kSceneStepMaxBodies = 1024; // fused per-scene step: bodies per scene, at most
+constexpr int kSceneStepMaxBodies = 1024; // fused per-scene worlds: bodies per scene, at most
+constexpr int kSceneStepBodies = 24;     // fused per-scene step: larger scenes take the staged kernels
 
 // EPA capacities. Vertices: the GJK tetrahedron plus one support per EPA iteration (at most
 // 65, code/nans.cpp:804). Faces grow by two per iteration on a convex polytope, but the
@@ -106,8 +107,19 @@ size_t epa_block_bytes();
 size_t epa_giant_scratch_bytes();
 int giant_grid(int sm_count);
 int launch_narrow_big(cudaStream_t st, const DevWorld &w); // returns a cudaError_t
-void launch_narrow_tiny(int grid, cudaStream_t st, const DevWorld &w);
+// the entries of one pair-tier launch
+enum PairPart
+{
+    PAIRS_FRONT = 0, // what the GJK pass queued
+    PAIRS_BACK = 1,  // what the per-thread EPA left over
+    PAIRS_ALL = 2,   // every candidate, in place of the GJK and per-thread EPA passes
+};
+void launch_gjk(int grid, cudaStream_t st, const DevWorld &w);
+void launch_gjk_long(int grid, cudaStream_t st, const DevWorld &w);
+void launch_epa_tiny(cudaStream_t st, const DevWorld &w);
+void launch_pair_warp(cudaStream_t st, const DevWorld &w, int part);
 int epa_tiny_grid(int sm_count);   // resident blocks of the per-thread EPA on sm_count SMs
+int pair_warp_grid(int sm_count);  // resident blocks of the pair tier on sm_count SMs
 int narrow_kernel_attrs();         // per-device kernel attributes (cudaError_t), set at world creation
 int large_kernel_attrs();
 void launch_epa_medium(cudaStream_t st, const DevWorld &w);
