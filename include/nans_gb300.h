@@ -376,7 +376,7 @@ int nans_render_scene(nans_world *world, uint32_t scene, const float eye[3], con
  *   d_angular_velocity hold nbodies x 3 floats, d_mass and d_moi nbodies floats; velocities
  *   are updated in place. floor (host) holds Position[3], V[3], W[3], Mass, MOI of the static
  *   ground; d_pairs holds npairs contact records as nans_get_pairs returns them.
- * Scratch lives in one fixed device array inside the library (about 2.7 MB on every GPU that
+ * Scratch lives in one fixed device array inside the library (about 2.5 MB on every GPU that
  * loads it, kept until the process exits): at most 16,384 bodies and 16,384 contacts per call,
  * larger requests fail with NANS_ERR_INVALID_ARGUMENT. Every call shares that array, so calls
  * whose kernels overlap on the GPU race; serialise them. The first call on a device (and the
