@@ -9,7 +9,7 @@
 // number wave = 1 + max(last wave of body A, last wave of body B); contacts of one wave run
 // in parallel and waves run in order, which reproduces the sequential result bit for bit.
 #pragma once
-#include "nans_fbound.cuh"
+#include "nans_impulse.cuh"
 #include "nans_kernels.cuh"
 
 namespace nans
@@ -208,8 +208,12 @@ __device__ __forceinline__ void contact_apply(const DevWorld &w, int4 id, const 
             st2 = e.z;
         }
     }
+    // From zero sums the loop's last round follows from the increments (nans_impulse.cuh) but for one
+    // contact in a few thousand, near the friction cone's edge.
+    if (WARM || !impulse_direct((-jdvn + bias) * jn, (-jdvt1) * jt1, (-jdvt2) * jt2, c2, fb, iters, dn, dt1, dt2))
     {
         const float sn0 = sn, st10 = st1, st20 = st2;
+        dn = dt1 = dt2 = 0.0f;
         if (!(fb.ok && impulse_loop<true>(jdvn, jdvt1, jdvt2, bias, jn, jt1, jt2, c2, fb, iters, sn, st1, st2, dn, dt1,
                                           dt2)))
         {

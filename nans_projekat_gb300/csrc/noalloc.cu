@@ -338,8 +338,7 @@ __global__ void __launch_bounds__(kThreads) k_solve_static(unsigned *scratch, Bo
             const float jdvt2 = dot3(((V1 + cross3(W1, t2)) - V2) - cross3(W2, t2), t2);
             const float bias = q3.w + cr * jdvn;
             float sn = 0.0f, st1 = 0.0f, st2 = 0.0f, dn = 0.0f, dt1 = 0.0f, dt2 = 0.0f;
-            if (!(fb.ok && nans::impulse_loop<true>(jdvn, jdvt1, jdvt2, bias, jn, jt1, jt2, c2, fb, iters, sn, st1, st2,
-                                                    dn, dt1, dt2)))
+            if (!nans::impulse_direct((-jdvn + bias) * jn, (-jdvt1) * jt1, (-jdvt2) * jt2, c2, fb, iters, dn, dt1, dt2))
             {
                 sn = st1 = st2 = dn = dt1 = dt2 = 0.0f;
                 nans::impulse_loop<false>(jdvn, jdvt1, jdvt2, bias, jn, jt1, jt2, c2, fb, iters, sn, st1, st2, dn, dt1,
