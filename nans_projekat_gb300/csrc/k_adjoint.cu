@@ -48,7 +48,7 @@ __global__ void k_tape_copy(DevWorld w, TapeStep t)
         t.type[j] = w.cand_meta[c] & 7;
 #pragma unroll
         for (int q = 0; q < 9; ++q)
-            t.k[(size_t)9 * j + q] = w.s_k[(size_t)9 * j + q];
+            t.k[(size_t)9 * j + q] = *slot_k(w, q, j);
         t.fwd[2 * (size_t)j] = w.s_fwd[2 * (size_t)c];
         t.fwd[2 * (size_t)j + 1] = w.s_fwd[2 * (size_t)c + 1];
     }

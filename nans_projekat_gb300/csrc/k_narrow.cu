@@ -468,6 +468,48 @@ __device__ int epa_run(const DevWorld &w, B &E, const Shape &A, const Shape &Bs,
 }
 
 
+// GJK and the per-thread EPA run as separate kernels. The GJK pass keeps its registers low
+// and its code small; a hit's final simplex (4 x (P, SupA, SupB), 36 floats) goes to the
+// candidate's solver-constant slot (s_k, 9 float4, written only later by the solver) and the
+// candidate to a compact queue (s_order, likewise free until the solver), so the EPA pass runs
+// only hits, every lane on an EPA.
+__device__ __forceinline__ void store_simplex(const DevWorld &w, int c, const GV &s0, const GV &s1, const GV &s2,
+                                              const GV &s3)
+{
+    *slot_k(w, 0, c) = make_float4(s0.p.x, s0.p.y, s0.p.z, s0.sa.x);
+    *slot_k(w, 1, c) = make_float4(s0.sa.y, s0.sa.z, s0.sb.x, s0.sb.y);
+    *slot_k(w, 2, c) = make_float4(s0.sb.z, s1.p.x, s1.p.y, s1.p.z);
+    *slot_k(w, 3, c) = make_float4(s1.sa.x, s1.sa.y, s1.sa.z, s1.sb.x);
+    *slot_k(w, 4, c) = make_float4(s1.sb.y, s1.sb.z, s2.p.x, s2.p.y);
+    *slot_k(w, 5, c) = make_float4(s2.p.z, s2.sa.x, s2.sa.y, s2.sa.z);
+    *slot_k(w, 6, c) = make_float4(s2.sb.x, s2.sb.y, s2.sb.z, s3.p.x);
+    *slot_k(w, 7, c) = make_float4(s3.p.y, s3.p.z, s3.sa.x, s3.sa.y);
+    *slot_k(w, 8, c) = make_float4(s3.sa.z, s3.sb.x, s3.sb.y, s3.sb.z);
+}
+__device__ __forceinline__ void load_simplex(const DevWorld &w, int c, GV &s0, GV &s1, GV &s2, GV &s3)
+{
+    const float4 k0 = *slot_k(w, 0, c), k1 = *slot_k(w, 1, c), k2 = *slot_k(w, 2, c), k3 = *slot_k(w, 3, c),
+                 k4 = *slot_k(w, 4, c), k5 = *slot_k(w, 5, c), k6 = *slot_k(w, 6, c), k7 = *slot_k(w, 7, c),
+                 k8 = *slot_k(w, 8, c);
+    s0.p = mk3(k0.x, k0.y, k0.z);
+    s0.sa = mk3(k0.w, k1.x, k1.y);
+    s0.sb = mk3(k1.z, k1.w, k2.x);
+    s1.p = mk3(k2.y, k2.z, k2.w);
+    s1.sa = mk3(k3.x, k3.y, k3.z);
+    s1.sb = mk3(k3.w, k4.x, k4.y);
+    s2.p = mk3(k4.z, k4.w, k5.x);
+    s2.sa = mk3(k5.y, k5.z, k5.w);
+    s2.sb = mk3(k6.x, k6.y, k6.z);
+    s3.p = mk3(k6.w, k7.x, k7.y);
+    s3.sa = mk3(k7.z, k7.w, k8.x);
+    s3.sb = mk3(k8.y, k8.z, k8.w);
+}
+// Float e (0..35, vertex by vertex) of candidate c's simplex.
+__device__ __forceinline__ float *simplex_at(const DevWorld &w, int c, int e)
+{
+    return reinterpret_cast<float *>(slot_k(w, e >> 2, c)) + (e & 3);
+}
+
 constexpr int kPairThreads = 64;
 
 // Returns the tier-3 queue index (the caller may leave its state in handover[q]), or -1.
@@ -676,7 +718,7 @@ __device__ __forceinline__ v3 box_support(const Verts8 &r, v3 d)
 // ResolveCollision (code/nans.cpp:787-904) by one thread; same results as epa_run and epa_warp,
 // or EPA_OVERFLOW for a polytope it does not hold: one that outgrows it, has a repeated or NaN
 // vertex, or loses every face.
-// `simp` is the GJK simplex as the GJK pass stored it (4 x (P, SupA, SupB), 36 floats).
+// The simplex is candidate c's, as the GJK pass stored it.
 // Every running EPA of a warp is at the same iteration and a regular polytope has 4 + 2 it faces,
 // so the face loop is uniform; it only marks the visible faces, whose edges (one or two faces in
 // 97 % of the iterations) then follow in a loop of their own. With the edges inside the face loop
@@ -684,8 +726,8 @@ __device__ __forceinline__ v3 box_support(const Verts8 &r, v3 d)
 // The closest-face search of the next iteration is folded into the face loop and the face
 // creation: a running minimum with strict '<' over the kept faces, then the new ones, in list
 // order, is the reference's scan (a NaN first distance keeps face 0, as its scan does).
-__device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, const Shape &B, const float *simp,
-                        v3 &out_pa, v3 &out_pb, v3 &out_n, int &iters)
+__device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, const Shape &B, int c, v3 &out_pa,
+                        v3 &out_pb, v3 &out_n, int &iters)
 {
     TinyLocal L;
     const bool ra = A.npts == 8, rb = B.npts == 8;
@@ -695,15 +737,12 @@ __device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, c
     if (rb)
         load_verts8(w.verts, B.off, VB);
     bool distinct = true;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
     {
-        const float *q = simp + 9 * i;
-        GV g;
-        g.p = mk3(q[0], q[1], q[2]);
-        g.sa = mk3(q[3], q[4], q[5]);
-        g.sb = mk3(q[6], q[7], q[8]);
-        distinct = tiny_put(S, L, t, i, g) && distinct;
+        GV g[4];
+        load_simplex(w, c, g[0], g[1], g[2], g[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            distinct = tiny_put(S, L, t, i, g[i]) && distinct;
     }
     if (!distinct)
         return EPA_OVERFLOW;
@@ -833,26 +872,6 @@ __device__ int epa_tiny(const DevWorld &w, TinySmem &S, int t, const Shape &A, c
         cs = ncs;
     }
     return EPA_NONE;
-}
-
-// GJK and the per-thread EPA run as separate kernels. The GJK pass keeps its registers low
-// and its code small; a hit's final simplex (4 x (P, SupA, SupB), 36 floats) goes to the
-// candidate's solver-constant slot (s_k, 9 float4, written only later by the solver) and the
-// candidate to a compact queue (s_order, likewise free until the solver), so the EPA pass runs
-// only hits, every lane on an EPA.
-__device__ __forceinline__ void store_simplex(const DevWorld &w, int c, const GV &s0, const GV &s1, const GV &s2,
-                                              const GV &s3)
-{
-    float4 *o = w.s_k + 9 * (size_t)c;
-    o[0] = make_float4(s0.p.x, s0.p.y, s0.p.z, s0.sa.x);
-    o[1] = make_float4(s0.sa.y, s0.sa.z, s0.sb.x, s0.sb.y);
-    o[2] = make_float4(s0.sb.z, s1.p.x, s1.p.y, s1.p.z);
-    o[3] = make_float4(s1.sa.x, s1.sa.y, s1.sa.z, s1.sb.x);
-    o[4] = make_float4(s1.sb.y, s1.sb.z, s2.p.x, s2.p.y);
-    o[5] = make_float4(s2.p.z, s2.sa.x, s2.sa.y, s2.sa.z);
-    o[6] = make_float4(s2.sb.x, s2.sb.y, s2.sb.z, s3.p.x);
-    o[7] = make_float4(s3.p.y, s3.p.z, s3.sa.x, s3.sa.y);
-    o[8] = make_float4(s3.sa.z, s3.sb.x, s3.sb.y, s3.sb.z);
 }
 
 // The pair tier's queue entries (long_cand): candidate and state. An unfinished GJK run is
@@ -1021,21 +1040,8 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk_long(DevWorld w)
         const int2 q = w.long_cand[i];
         if (q.y == kPairEpa || !dev_check(w, q.x >= 0 && q.x < w.cand_cap, 16, q.x, w.cand_cap))
             continue;
-        const float4 *o = w.s_k + 9 * (size_t)q.x;
-        const float4 k0 = o[0], k1 = o[1], k2 = o[2], k3 = o[3], k4 = o[4], k5 = o[5], k6 = o[6], k7 = o[7], k8 = o[8];
         GV s0, s1, s2, s3;
-        s0.p = mk3(k0.x, k0.y, k0.z);
-        s0.sa = mk3(k0.w, k1.x, k1.y);
-        s0.sb = mk3(k1.z, k1.w, k2.x);
-        s1.p = mk3(k2.y, k2.z, k2.w);
-        s1.sa = mk3(k3.x, k3.y, k3.z);
-        s1.sb = mk3(k3.w, k4.x, k4.y);
-        s2.p = mk3(k4.z, k4.w, k5.x);
-        s2.sa = mk3(k5.y, k5.z, k5.w);
-        s2.sb = mk3(k6.x, k6.y, k6.z);
-        s3.p = mk3(k6.w, k7.x, k7.y);
-        s3.sa = mk3(k7.z, k7.w, k8.x);
-        s3.sb = mk3(k8.y, k8.z, k8.w);
+        load_simplex(w, q.x, s0, s1, s2, s3);
         int np = q.y & 0xff, it = q.y >> 8;
         bool hull;
         const bool hit = gjk_run(w, q.x, w.cand_a[q.x], w.cand_b[q.x], 65, s0, s1, s2, s3, np, it, hull) == G_FOUND;
@@ -1197,8 +1203,7 @@ __global__ void __launch_bounds__(kTinyThreads, 8) k_epa_tiny(DevWorld w)
         const Shape A = load_shape(w, w.cand_a[c]), B = load_shape(w, w.cand_b[c]);
         v3 pa, pb, nn;
         int iters = 0;
-        const int r =
-            epa_tiny(w, S, t, A, B, reinterpret_cast<const float *>(w.s_k + 9 * (size_t)c), pa, pb, nn, iters);
+        const int r = epa_tiny(w, S, t, A, B, c, pa, pb, nn, iters);
         if (r != EPA_OVERFLOW)
         {
             const int pidx = w.cand_pidx[c];
@@ -1216,10 +1221,9 @@ __global__ void __launch_bounds__(kTinyThreads, 8) k_epa_tiny(DevWorld w)
 __device__ __forceinline__ int pair_warp(const DevWorld &w, WarpEpa &S, int c, bool gjk, int n, int it, int lane)
 {
     const Shape A = load_shape(w, w.cand_a[c]), B = load_shape(w, w.cand_b[c]);
-    float *sq = reinterpret_cast<float *>(w.s_k + 9 * (size_t)c); // 36 floats, vertex by vertex
     const v3 va = lane_vertex(w.verts, A, lane), vb = lane_vertex(w.verts, B, lane);
     for (int k = lane; k < 9 * n; k += 32)
-        S.v[k % 9][k / 9] = sq[k];
+        S.v[k % 9][k / 9] = *simplex_at(w, c, k);
     __syncwarp();
     if (gjk)
     {
@@ -1230,7 +1234,7 @@ __device__ __forceinline__ int pair_warp(const DevWorld &w, WarpEpa &S, int c, b
             return EPA_NONE;
         }
         for (int k = lane; k < 36; k += 32)
-            sq[k] = S.v[k % 9][k / 9]; // for the later tiers
+            *simplex_at(w, c, k) = S.v[k % 9][k / 9]; // for the later tiers
     }
     v3 pa, pb, nn;
     int iters = 0;
@@ -1300,14 +1304,8 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32) k_epa_medium(
             break;
         const int cc = w.med_cand[q];
         const Shape A = load_shape(w, w.cand_a[cc]), B = load_shape(w, w.cand_b[cc]);
-        const float *sq = reinterpret_cast<const float *>(w.s_k + 9 * (size_t)cc);
         GV g[4];
-        for (int i = 0; i < 4; ++i)
-        {
-            g[i].p = mk3(sq[9 * i], sq[9 * i + 1], sq[9 * i + 2]);
-            g[i].sa = mk3(sq[9 * i + 3], sq[9 * i + 4], sq[9 * i + 5]);
-            g[i].sb = mk3(sq[9 * i + 6], sq[9 * i + 7], sq[9 * i + 8]);
-        }
+        load_simplex(w, cc, g[0], g[1], g[2], g[3]);
         v3 pa, pb, nn;
         int4 ovf;
         int r = epa_run(w, E, A, B, g[0], g[1], g[2], g[3], pa, pb, nn, lane, ovf);
@@ -1470,14 +1468,8 @@ __global__ void __launch_bounds__(kSceneThreads) k_scene_step(DevWorld w, float 
             if (cc < 0)
                 continue;
             const Shape A = load_shape(w, w.cand_a[cc]), B = load_shape(w, w.cand_b[cc]);
-            const float *sq = reinterpret_cast<const float *>(w.s_k + 9 * (size_t)cc);
             GV g[4];
-            for (int v = 0; v < 4; ++v)
-            {
-                g[v].p = mk3(sq[9 * v], sq[9 * v + 1], sq[9 * v + 2]);
-                g[v].sa = mk3(sq[9 * v + 3], sq[9 * v + 4], sq[9 * v + 5]);
-                g[v].sb = mk3(sq[9 * v + 6], sq[9 * v + 7], sq[9 * v + 8]);
-            }
+            load_simplex(w, cc, g[0], g[1], g[2], g[3]);
             v3 pa, pb, nn;
             int4 ovf;
             const int r = epa_run(w, E, A, B, g[0], g[1], g[2], g[3], pa, pb, nn, lane, ovf);

@@ -132,7 +132,9 @@ struct DevWorld
     int4 *s_ids;                        // per solve slot (wave order): candidate, body A,
                                         // body B (-1 - B when B is the floor), pair-space index
     float4 *s_k;                        // per solve slot: 9 float4 of contact constants; during
-                                        // the narrowphase, per candidate: the GJK simplex of a hit
+                                        // the narrowphase, per candidate: the GJK simplex of a hit.
+                                        // Field by field (slot_k): the slots of neighbouring
+                                        // threads lie side by side
     int *s_last;                        // per body: last wave touching it
     int solve_cache;                    // scenes of up to this many bodies solve their waves on
                                         // a shared-memory copy of their velocities
@@ -184,6 +186,14 @@ __device__ __forceinline__ v3 hull_support(const float *__restrict__ verts, int 
 __device__ __forceinline__ v3 sphere_support(v3 p, float radius, v3 d)
 {
     return p + radius * normalize3(d);
+}
+
+// Float4 q of slot (or candidate) i. Nine rows of cand_cap: a warp's 32 slots are 512 contiguous bytes
+// a row, where records of 144 bytes touched 32 cache lines per load (36 loads of four bytes each in
+// the per-thread EPA).
+__device__ __forceinline__ float4 *slot_k(const DevWorld &w, int q, int i)
+{
+    return w.s_k + (size_t)q * w.cand_cap + i;
 }
 
 struct Shape

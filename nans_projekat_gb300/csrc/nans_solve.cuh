@@ -146,8 +146,8 @@ __device__ __forceinline__ bool impulse_loop(float jdvn, float jdvt1, float jdvt
 // normal / tangent velocities, the applied impulses and the active set of the closed form
 // (normal impulse max(Ln, 0), tangent impulses clamp(Lt, -mu*Ln, mu*Ln)).
 //
-// id = the slot's (candidate, body A, body B or -1 - B for the floor, pair-space index), kp its
-// constants, hd their first part (read a wave ahead), vel / omg the velocities (the scene's
+// id = the slot's (candidate, body A, body B or -1 - B for the floor, pair-space index), hd the
+// first part of its constants (read a wave ahead), vel / omg the velocities (the scene's
 // shared-memory copy or the world's arrays) at ia / ib.
 // The iteration loop's operands (N, T1, T2 with their effective masses, and the Baumgarte
 // term), read a wave ahead; the rest of the record is read at the wave's start and needed after
@@ -159,18 +159,18 @@ struct KHead
     float4 n, t1, t2; // (N, Jn), (T1, Jt1), (T2, Jt2)
     float bias0;
 };
-__device__ __forceinline__ KHead load_head(const float4 *kp)
+__device__ __forceinline__ KHead load_head(const DevWorld &w, int slot)
 {
     KHead h;
-    h.n = kp[0];
-    h.t1 = kp[1];
-    h.t2 = kp[2];
-    h.bias0 = reinterpret_cast<const float *>(kp + 3)[3];
+    h.n = *slot_k(w, 0, slot);
+    h.t1 = *slot_k(w, 1, slot);
+    h.t2 = *slot_k(w, 2, slot);
+    h.bias0 = slot_k(w, 3, slot)->w;
     return h;
 }
 
 template <bool WARM>
-__device__ __forceinline__ void contact_apply(const DevWorld &w, int4 id, const KHead &hd, const float4 *kp,
+__device__ __forceinline__ void contact_apply(const DevWorld &w, int4 id, const KHead &hd, int slot,
                                               float4 *vel, float4 *omg, int ia, int ib, float cr, float cf,
                                               double c2, const FBound &fb, int iters)
 {
@@ -179,7 +179,7 @@ __device__ __forceinline__ void contact_apply(const DevWorld &w, int4 id, const 
     float4 k[9];
 #pragma unroll
     for (int q = 3; q < 9; ++q)
-        k[q] = kp[q];
+        k[q] = *slot_k(w, q, slot);
     k[0] = hd.n;
     k[1] = hd.t1;
     k[2] = hd.t2;
@@ -480,7 +480,7 @@ __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, 
         contact_constants(w, c, a, b, dt, k);
 #pragma unroll
         for (int q = 0; q < 9; ++q)
-            w.s_k[(size_t)9 * pos + q] = k[q];
+            *slot_k(w, q, pos) = k[q];
         w.s_ids[pos] = make_int4(c, a, b >= w.n_dyn ? -1 - b : b, w.cand_pidx ? w.cand_pidx[c] : 0);
     }
     __threadfence_block();
@@ -527,7 +527,7 @@ __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, 
         if (i < hi && !have)
         {
             id = w.s_ids[cb + i];
-            hd = load_head(w.s_k + (size_t)9 * (cb + i));
+            hd = load_head(w, cb + i);
         }
         else if (i >= hi)
         {
@@ -536,7 +536,7 @@ __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, 
             if (next_wave)
             {
                 id = w.s_ids[cb + hi + tid];
-                hd = load_head(w.s_k + (size_t)9 * (cb + hi + tid));
+                hd = load_head(w, cb + hi + tid);
             }
         }
         while (i < hi)
@@ -549,11 +549,11 @@ __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, 
             if (nx_ok)
             {
                 idn = w.s_ids[cb + nx];
-                hdn = load_head(w.s_k + (size_t)9 * (cb + nx));
+                hdn = load_head(w, cb + nx);
             }
             const int b = id.z >= 0 ? id.z : -1 - id.z;
             const int ib = (cached && id.z < 0) ? nb : b - off;
-            contact_apply<WARM>(w, id, hd, w.s_k + (size_t)9 * (cb + i), vel, omg, id.y - off, ib, cr, cf, c2, fb,
+            contact_apply<WARM>(w, id, hd, cb + i, vel, omg, id.y - off, ib, cr, cf, c2, fb,
                                 iters);
             id = idn;
             hd = hdn;
