@@ -67,7 +67,7 @@ struct nans_world
     int n_scenes = 0, n_dyn = 0, n_all = 0, n_cubes = 0, n_spheres = 0;
     long long pair_total = 0;
     int cand_cap = 0;
-    int cull_blocks = 0;    // one thread per pair-mask word
+    int cull_blocks = 0;    // blocks of the cull's placement
     int max_scene_bodies = 0;
 
     std::vector<void *> allocs;     // per-upload device buffers
@@ -438,7 +438,8 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     }
     w->pair_total = pair_acc;
     w->max_scene_bodies = max_bodies;
-    w->cull_blocks = (int)((word_acc + kCullThreads - 1) / kCullThreads);
+    const long long cull_words = kCullThreads * cull_words_per_thread((int)word_acc, w->sm_count);
+    w->cull_blocks = (int)((word_acc + cull_words - 1) / cull_words);
 
     DevWorld &d = w->dw;
     d = DevWorld{};
@@ -448,6 +449,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     d.n_all = nall;
     d.pair_total = pair_acc;
     d.n_words = (int)word_acc;
+    d.cull_blocks = w->cull_blocks;
     d.n_tiles = (int)tiles.size();
     auto &L = w->allocs;
     int rc;
@@ -470,7 +472,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
         (rc = dalloc(w, L, &d.pair_mask, (size_t)word_acc)) || (rc = dalloc(w, L, &p_wscene, (size_t)word_acc)) ||
         (rc = dalloc(w, L, &p_tiles, tiles.size())) || (rc = dalloc(w, L, &p_rest, rest_tasks.size())) ||
         (rc = dalloc(w, L, &d.epa_hist, (size_t)word_acc * 32)) ||
-        (rc = dalloc(w, L, &d.block_hits, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.cull_total, 1)) ||
+        (rc = dalloc(w, L, &d.cull_state, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.cull_total, 1)) ||
         (rc = dalloc(w, L, &d.cull_max, 1)) ||
         (rc = dalloc(w, L, &d.n_cand, 1)) ||
         (rc = dalloc(w, L, &d.cand_begin, S)) || (rc = dalloc(w, L, &d.cand_end, S)) ||
@@ -626,39 +628,45 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     return NANS_OK;
 }
 
-// Enqueues the cull (three kernels) on the world's stream.
-// The culled pair mask and its per-block counts (the scan's input): by tiles (cube-cube pairs
-// 32 x 32 per warp, the other pairs per scene, then the counts), or one lane per pair
-// (k_cull_mask: the all-pairs mode, and the tuning's alternative). The same mask either way.
-void enqueue_cull_mask(nans_world *w)
+// Whether the cull's blocks make their mask words themselves, one lane per pair: the all-pairs mode and
+// the tuning's alternative. (The tiles are the faster ones at every size: 91 against 101 us a step at
+// 536 words, 225 against 234 at 119,000.)
+bool cull_by_lane(const nans_world *w) { return (w->flags & NANS_WORLD_ALL_PAIRS) || !w->cull_tiles; }
+
+// The tiles' mask is cleared by the sweep, or where that would be many words a body by a memset.
+bool sweep_clears_mask(const nans_world *w)
+{
+    return !cull_by_lane(w) && w->dw.n_words / 128 <= w->n_all;
+}
+
+// Enqueues a step's sweep, which also clears what the step counts.
+void enqueue_sweep(nans_world *w, float pending_dt, float dt, int flags)
+{
+    flags |= SW_STEP_START | (sweep_clears_mask(w) ? SW_CLEAR_MASK : 0);
+    k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, w->stream>>>(w->dw, pending_dt, dt, flags);
+}
+
+// Enqueues the cull on the world's stream: the mask by tiles (cube-cube pairs 32 x 32 per warp, the
+// other pairs in chunks), then the candidates at their places; or the latter alone.
+void enqueue_cull(nans_world *w)
 {
     cudaStream_t st = w->stream;
     const int all_pairs = (w->flags & NANS_WORLD_ALL_PAIRS) ? 1 : 0;
     if (w->cull_blocks <= 0)
-        return;
-    if (all_pairs || !w->cull_tiles)
     {
-        k_cull_mask<<<w->cull_blocks, kCullThreads, 0, st>>>(w->dw, all_pairs);
+        cudaMemsetAsync(w->dw.n_cand, 0, sizeof(int), st);
+        cudaMemsetAsync(w->dw.cull_total, 0, sizeof(int), st);
         return;
     }
-    const int per_block = kCullTileThreads / 32, cap = 8 * w->sm_count;
-    cudaMemsetAsync(w->dw.pair_mask, 0, (size_t)w->dw.n_words * sizeof(unsigned), st);
-    if (w->dw.n_tiles > 0)
-        k_cull_tiles<<<std::min(cap, (w->dw.n_tiles + per_block - 1) / per_block), kCullTileThreads, 0, st>>>(w->dw);
-    if (w->dw.n_rest_tasks > 0)
-        k_cull_rest<<<std::min(cap, (w->dw.n_rest_tasks + per_block - 1) / per_block), kCullTileThreads, 0, st>>>(
-            w->dw);
-    k_cull_count<<<w->cull_blocks, kCullThreads, 0, st>>>(w->dw);
-}
-
-// Enqueues the cull on the world's stream: mask, scan, ordered write.
-void enqueue_cull(nans_world *w)
-{
-    cudaStream_t st = w->stream;
-    enqueue_cull_mask(w);
-    k_cull_scan<<<1, 1024, 0, st>>>(w->dw, w->cull_blocks);
-    if (w->cull_blocks > 0)
-        k_cull_write<<<w->cull_blocks, kCullThreads, 0, st>>>(w->dw);
+    const bool by_lane = cull_by_lane(w);
+    if (!by_lane)
+    {
+        const long long warps = (long long)w->dw.n_tiles + w->dw.n_rest_tasks, per = kCullTileThreads / 32;
+        if (!sweep_clears_mask(w))
+            cudaMemsetAsync(w->dw.pair_mask, 0, (size_t)w->dw.n_words * sizeof(unsigned), st);
+        k_cull_tiles<<<(int)std::min<long long>(8 * w->sm_count, (warps + per - 1) / per), kCullTileThreads, 0, st>>>(w->dw);
+    }
+    launch_cull_place(w->dw, by_lane, all_pairs, st);
 }
 
 // GJK and the EPA tiers of every pair that does not outgrow the pair tier, on the world's stream;
@@ -782,8 +790,7 @@ cudaError_t enqueue_fused(nans_world *w, float pending_dt, float dt, int flags)
 {
     cudaStream_t st = w->stream;
     DevWorld &d = w->dw;
-    k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(d, pending_dt, dt,
-                                                                                       flags | SW_CLEAR_COUNTERS);
+    enqueue_sweep(w, pending_dt, dt, flags);
     launch_scene_step(d, solve_smem(w), dt, (w->flags & NANS_WORLD_ALL_PAIRS) ? 1 : 0, st, 0, 0);
     return enqueue_fused_tail(w, dt, st);
 }
@@ -808,8 +815,7 @@ cudaError_t enqueue_fused_conditional(nans_world *w, float pending_dt, float dt,
     cudaGraphConditionalHandle h = 0;
     if ((e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
         return e;
-    k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(d, pending_dt, dt,
-                                                                                       flags | SW_CLEAR_COUNTERS);
+    enqueue_sweep(w, pending_dt, dt, flags);
     launch_scene_step(d, solve_smem(w), dt, (w->flags & NANS_WORLD_ALL_PAIRS) ? 1 : 0, st, h, 1);
     if ((e = cudaGetLastError()) != cudaSuccess)
         return e;
@@ -848,12 +854,7 @@ int step_eager(nans_world *w, float dt, bool check_capacity)
         after_step(w, dt);
         return NANS_OK;
     }
-    CK(cudaMemsetAsync(d.work_counter, 0, kWorkCounters * sizeof(int), st));
-    CK(cudaMemsetAsync(d.cand_begin, 0, w->n_scenes * sizeof(int), st));
-    CK(cudaMemsetAsync(d.cand_end, 0, w->n_scenes * sizeof(int), st));
-    CK(cudaMemsetAsync(d.scene_late, 0, w->n_scenes * sizeof(int), st));
-    k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(d, w->pending_dt, dt,
-                                                                                       sweep_flags(w));
+    enqueue_sweep(w, w->pending_dt, dt, sweep_flags(w));
     enqueue_cull(w);
     CK(cudaGetLastError());
     if (check_capacity)
@@ -870,8 +871,11 @@ int step_eager(nans_world *w, float dt, bool check_capacity)
             int rc = alloc_candidates(w, (int)std::min<long long>((long long)total + total / 4 + 1024, INT32_MAX / 16));
             if (rc)
                 return rc;
-            // the block counts were turned into offsets by the scan: count again
             CK(cudaMemsetAsync(d.status, 0, sizeof(unsigned), st));
+            // what the sweep cleared for the first try
+            CK(cudaMemsetAsync(d.work_counter, 0, kWorkCounters * sizeof(int), st));
+            CK(cudaMemsetAsync(d.cull_state, 0, w->cull_blocks * sizeof(unsigned long long), st));
+            CK(cudaMemsetAsync(d.pair_mask, 0, (size_t)d.n_words * sizeof(unsigned), st));
             enqueue_cull(w);
             CK(cudaGetLastError());
         }
@@ -942,12 +946,7 @@ int capture_steps(nans_world *w, float dt, int gsteps, cudaGraphExec_t *exec, fl
                 enqueue_fused(w, pdt, dt, fl);
             continue;
         }
-        cudaMemsetAsync(d.work_counter, 0, kWorkCounters * sizeof(int), st);
-        cudaMemsetAsync(d.cand_begin, 0, w->n_scenes * sizeof(int), st);
-        cudaMemsetAsync(d.cand_end, 0, w->n_scenes * sizeof(int), st);
-        cudaMemsetAsync(d.scene_late, 0, w->n_scenes * sizeof(int), st);
-        k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(
-            d, i == 0 ? pdt0 : dt, dt, i == 0 ? flags0 : (SW_INTEGRATE | SW_APPLY_VEL));
+        enqueue_sweep(w, i == 0 ? pdt0 : dt, dt, i == 0 ? flags0 : (SW_INTEGRATE | SW_APPLY_VEL));
         enqueue_cull(w);
         enqueue_narrow_solve(w, dt, nullptr);
     }
@@ -2077,13 +2076,8 @@ int nans_profile_steps(nans_world *w, float dt, uint32_t nsteps, float *stage_ms
     DevWorld &d = w->dw;
     for (uint32_t k = 0; k < nsteps; ++k)
     {
-        CK(cudaMemsetAsync(d.work_counter, 0, kWorkCounters * sizeof(int), st));
-        CK(cudaMemsetAsync(d.cand_begin, 0, w->n_scenes * sizeof(int), st));
-        CK(cudaMemsetAsync(d.cand_end, 0, w->n_scenes * sizeof(int), st));
-        CK(cudaMemsetAsync(d.scene_late, 0, w->n_scenes * sizeof(int), st));
         CK(cudaEventRecord(ev[0], st));
-        k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(d, w->pending_dt, dt,
-                                                                                           sweep_flags(w));
+        enqueue_sweep(w, w->pending_dt, dt, sweep_flags(w));
         CK(cudaEventRecord(ev[1], st));
         enqueue_cull(w);
         CK(cudaEventRecord(ev[2], st));
@@ -2132,12 +2126,7 @@ int nans_profile_timeline(nans_world *w, float dt, uint32_t nsteps, float *t_ms)
     for (uint32_t k = 0; k < nsteps; ++k)
     {
         CK(cudaEventRecord(ev[0], st));
-        CK(cudaMemsetAsync(d.work_counter, 0, kWorkCounters * sizeof(int), st));
-        CK(cudaMemsetAsync(d.cand_begin, 0, w->n_scenes * sizeof(int), st));
-        CK(cudaMemsetAsync(d.cand_end, 0, w->n_scenes * sizeof(int), st));
-        CK(cudaMemsetAsync(d.scene_late, 0, w->n_scenes * sizeof(int), st));
-        k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(d, w->pending_dt, dt,
-                                                                                           sweep_flags(w));
+        enqueue_sweep(w, w->pending_dt, dt, sweep_flags(w));
         CK(cudaEventRecord(ev[1], st));
         enqueue_cull(w);
         CK(cudaEventRecord(ev[2], st));

@@ -132,8 +132,22 @@ __device__ __forceinline__ void store_box(const DevWorld &w, int b, v3 lo, v3 hi
 __global__ void k_sweep(DevWorld w, float pending_dt, float dt, int flags)
 {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((flags & SW_CLEAR_COUNTERS) && b < kWorkCounters)
-        w.work_counter[b] = 0;
+    if (flags & SW_STEP_START)
+    {
+        if (b < kWorkCounters)
+            w.work_counter[b] = 0;
+        if (b < w.n_scenes)
+        {
+            w.cand_begin[b] = 0;
+            w.cand_end[b] = 0;
+            w.scene_late[b] = 0;
+        }
+        for (int i = b; i < w.cull_blocks; i += gridDim.x * blockDim.x)
+            w.cull_state[i] = 0ull;
+    }
+    if (flags & SW_CLEAR_MASK)
+        for (int i = b; i < w.n_words; i += gridDim.x * blockDim.x)
+            w.pair_mask[i] = 0u;
     if (b >= w.n_all)
         return;
     const bool is_floor = b >= w.n_dyn;

@@ -78,7 +78,8 @@ struct DevWorld
     int n_rest_tasks;
     const int *word_scene;              // scene of each mask word
     int n_words;
-    int *block_hits;                    // per cull block: culled pairs, then candidate offset
+    unsigned long long *cull_state;     // per cull block: what is known of its candidates
+    int cull_blocks;
     int *cull_total;                    // candidates before the capacity clamp
     int *cull_max;                      // largest cull_total since the host last cleared it
     int *cand_begin, *cand_end;         // per scene candidate range
@@ -88,7 +89,7 @@ struct DevWorld
     // narrowphase output, per candidate
     int *hit;
     float4 *c_pa, *c_pb, *c_n;
-    int *work_counter;                  // [0] narrowphase head, [1] solver head, [2] block-EPA
+    int *work_counter;                  // [0] narrowphase head, [1] cull block, [2] block-EPA
                                         // head, [3] block-EPA queue length, [5] warp-EPA queue
                                         // length, [6] warp-EPA head, [7] pair-tier queue length
                                         // (from the front) and [4] from the back,

@@ -14,7 +14,9 @@ enum SweepFlags
     SW_INTEGRATE = 2,   // RK4 + vertices + AABB
     SW_MODEL_INPUT = 4, // take Model from the uploaded records instead of rebuilding it
     SW_FORCES = 8,      // read (then clear) external forces and torques
-    SW_CLEAR_COUNTERS = 16, // zero the work counters first (the fused step, which has no memset)
+    SW_STEP_START = 16, // clear what the step counts and lists: work counters, per-scene candidate
+                        // ranges and late marks, the cull's block states
+    SW_CLEAR_MASK = 32, // clear the pair mask
 };
 
 // Global body ids of pair (type, i, j) of scene s whose cubes start at c0 (nc cubes).
@@ -30,8 +32,9 @@ __device__ __forceinline__ void pair_ids(const DevWorld &w, int s, int c0, int n
 }
 
 constexpr int kCullThreads = 256;
+constexpr int kCullList = 4096;  // candidates a block of the cull's placement lists at a time
 constexpr int kCullTileThreads = 256;
-constexpr int kRestChunksPerTask = 64; // 32-pair chunks of non-cube-cube pairs per cull task
+constexpr int kRestChunksPerTask = 8; // 32-pair chunks of non-cube-cube pairs per cull task
 constexpr int kSolveLateThreads = 128; // solver blocks of the second pass (late scenes)
 constexpr int kSolveLateBlocksPerSm = 6; // second-pass solver blocks per SM (registers allow six)
 constexpr int kWaveChunk = 256;     // solver: candidates compacted and labelled per chunk
@@ -94,12 +97,10 @@ __global__ void k_sincos(const float *x, float *s, float *c, int n);
 __global__ void k_state_in(DevWorld w, const float *stage, const int *body_rec, int n_cubes, int mask);
 __global__ void k_state_out(DevWorld w, float *stage, const int *body_rec, int n_cubes, int mask);
 
-__global__ void k_cull_mask(DevWorld w, int all_pairs);
-__global__ void k_cull_scan(DevWorld w, int nblocks);
-__global__ void k_cull_write(DevWorld w);
 __global__ void k_cull_tiles(DevWorld w);
-__global__ void k_cull_rest(DevWorld w);
-__global__ void k_cull_count(DevWorld w);
+// mask: the blocks make their mask words themselves
+int cull_words_per_thread(int n_words, int sm_count);
+void launch_cull_place(const DevWorld &w, int mask, int all_pairs, cudaStream_t st);
 
 int narrow_blocks_per_sm(int warps);
 size_t epa_big_bytes();

@@ -79,3 +79,28 @@ def test_hull_sizes(oracle_lib, npts, n_scenes):
     from nans_projekat_gb300 import scenes
     batch = [_hull_scene(scenes, npts, 5 + i) for i in range(n_scenes)]
     _compare(batch, 30, lambda w, n: w.batch_step(DT, n, 10))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_scenes,bodies", [(1, 92), (30, 75)])
+def test_full_blocks_of_the_cull(n_scenes, bodies):
+    """With every pair kept, a block of the cull's placement lists its candidates in more than one
+    round (8,192 pairs a block against a list of 4,096): the same contacts and states as the culled
+    run, for one block's pairs and for several blocks'."""
+    from nans_projekat_gb300 import lib, scenes
+    batch = scenes.stack_batch(n_scenes, seed=17, lo=bodies, hi=bodies)
+    out = []
+    for every in (False, True):
+        w = lib.World(all_pairs=every, max_candidates=2 * n_scenes * bodies * bodies)
+        w.upload_batch(batch)
+        w.batch_step(DT, 12, 6)
+        pairs = [w.pairs(i) for i in range(n_scenes)]
+        out.append((w.get_state_arrays(), pairs, w.counts(), w.status()))
+        w.close()
+    assert out[1][2][0] > 4096 * (1 if n_scenes == 1 else 10) and out[0][2][1] == out[1][2][1]
+    assert out[0][3] == 0 and out[1][3] == 0
+    for a, b in zip(out[0][0], out[1][0]):
+        assert canon(a) == canon(b)
+    for p, q in zip(out[0][1], out[1][1]):
+        for f in ("Type", "IndexA", "IndexB", "PointA", "PointB", "N"):
+            assert canon(p[f]) == canon(q[f])
