@@ -54,6 +54,8 @@ constexpr int kSweepThreads = 256;
 constexpr int kTuneSteps = 20;       // timed steps per autotuner candidate
 } // namespace
 
+constexpr size_t kHostStage = 64 * 1024; // bytes a world stages small downloads in
+
 struct nans_world
 {
     int device = 0;
@@ -80,6 +82,7 @@ struct nans_world
     float *d_pairs_out = nullptr;
     int pairs_out_cap = 0;
     int *h_words = nullptr; // page-locked: status word, counts read back after a step
+    unsigned char *h_stage = nullptr; // page-locked, kHostStage bytes: small downloads in one wait
     int *d_small = nullptr; // [0] pair count for k_pairs_out, [1] contact count
     float4 *d_snap = nullptr;
 
@@ -115,9 +118,16 @@ struct nans_world
     cudaGraphExec_t gexec_t = nullptr;  // differentiable rollout: graph of one steady taped step
     int gt_cfg = -1;
     float gt_dt = 0.0f;
-    cudaGraphExec_t gexec1 = nullptr;   // plain path: graph of one step
-    float g1_dt = 0.0f, g1_pdt = 0.0f;
-    int g1_flags = -1, g1_cfg = -1;
+    struct Graph1
+    {
+        cudaGraphExec_t exec = nullptr;
+        float dt = 0.0f, pdt = 0.0f;
+        int flags = -1, cfg = -1;
+    };
+    Graph1 g1[4];                       // plain path: graphs of one step, by its sweep flags
+    int g1_next = 0;                    // the one that is captured over next
+    float eager_dt = 0.0f;              // the last plain step that ran kernel by kernel
+    int eager_flags = -1;
     unsigned long long graph_steps_run = 0, eager_steps_run = 0; // nans_step / nans_batch_step
 
     // differentiable rollout: the tape lives in a chunked device arena reused across forwards
@@ -176,12 +186,13 @@ void drop_graph(nans_world *w)
         w->gexec_b = nullptr;
     }
     w->gb_cfg = -1;
-    if (w->gexec1)
+    for (auto &g : w->g1)
     {
-        cudaGraphExecDestroy(w->gexec1);
-        w->gexec1 = nullptr;
+        if (g.exec)
+            cudaGraphExecDestroy(g.exec);
+        g = nans_world::Graph1{};
     }
-    w->g1_cfg = -1;
+    w->eager_flags = -1;
     if (w->gexec_t)
     {
         cudaGraphExecDestroy(w->gexec_t);
@@ -900,10 +911,9 @@ int status_code(nans_world *w, unsigned status);
 
 int check_status(nans_world *w)
 {
-    unsigned status = 0;
-    CK(cudaMemcpyAsync(&status, w->dw.status, sizeof(unsigned), cudaMemcpyDeviceToHost, w->stream));
+    CK(cudaMemcpyAsync(w->h_words, w->dw.status, sizeof(unsigned), cudaMemcpyDeviceToHost, w->stream));
     CK(cudaStreamSynchronize(w->stream));
-    return status_code(w, status);
+    return status_code(w, (unsigned)w->h_words[0]);
 }
 
 int set_params_all(nans_world *w, const nans_step_params *p)
@@ -1028,34 +1038,60 @@ int ensure_graph(nans_world *w, float dt, int gsteps, cudaGraphExec_t *exec)
 }
 
 // A one-step graph for the world's current step flags (steady or not): the plain path and
-// one-step batched calls replay it; it is captured again when the flags, dt or the previous
-// step's dt change.
-int ensure_graph1(nans_world *w, float dt)
+// one-step batched calls replay it. The last four are kept: a host that writes the state between
+// calls alternates between the flags of the step after it and the steady ones, and a capture costs
+// as much as a small scene's step.
+int ensure_graph1(nans_world *w, float dt, cudaGraphExec_t *exec)
 {
     const int flags = sweep_flags(w);
     const float pdt = (flags & SW_APPLY_VEL) ? w->pending_dt : 0.0f;
-    if (w->gexec1 && w->g1_dt == dt && w->g1_pdt == pdt && w->g1_flags == flags && w->g1_cfg == cfg_id(w))
-        return NANS_OK;
-    w->g1_cfg = -1;
-    int rc = capture_steps(w, dt, 1, &w->gexec1, pdt, flags);
+    for (auto &g : w->g1)
+        if (g.exec && g.dt == dt && g.pdt == pdt && g.flags == flags && g.cfg == cfg_id(w))
+        {
+            *exec = g.exec;
+            return NANS_OK;
+        }
+    nans_world::Graph1 &g = w->g1[w->g1_next];
+    w->g1_next = (w->g1_next + 1) % 4;
+    g.cfg = -1;
+    const int rc = capture_steps(w, dt, 1, &g.exec, pdt, flags);
     if (rc)
         return rc;
-    w->g1_dt = dt;
-    w->g1_pdt = pdt;
-    w->g1_flags = flags;
-    w->g1_cfg = cfg_id(w);
+    g.dt = dt;
+    g.pdt = pdt;
+    g.flags = flags;
+    g.cfg = cfg_id(w);
+    *exec = g.exec;
     return NANS_OK;
 }
 
 // One step from a one-step graph.
 int step_graph1(nans_world *w, float dt)
 {
-    int rc = ensure_graph1(w, dt);
+    cudaGraphExec_t exec = nullptr;
+    const int rc = ensure_graph1(w, dt, &exec);
     if (rc)
         return rc;
-    CK(cudaGraphLaunch(w->gexec1, w->stream));
+    CK(cudaGraphLaunch(exec, w->stream));
     after_step(w, dt);
     ++w->graph_steps_run;
+    return NANS_OK;
+}
+
+// One step of the plain path: from a graph, but kernel by kernel for the first step after an upload or a
+// set_state (external forces, input Model) unless the last such step was alike: a frame loop that
+// hands its records over every frame replays a graph from its second frame on.
+int plain_step(nans_world *w, float dt)
+{
+    const int flags = sweep_flags(w);
+    if (!(flags & (SW_FORCES | SW_MODEL_INPUT)) || (flags == w->eager_flags && dt == w->eager_dt))
+        return step_graph1(w, dt);
+    const int rc = step_eager(w, dt, false);
+    if (rc)
+        return rc;
+    w->eager_flags = flags;
+    w->eager_dt = dt;
+    ++w->eager_steps_run;
     return NANS_OK;
 }
 
@@ -1168,19 +1204,8 @@ int plain_steps(nans_world *w, float dt, uint32_t nsteps)
         // The candidate buffers hold every pair of every scene, and the cull writes at most one
         // candidate per pair, so no step can overflow them: no copy aside, one status read.
         for (uint32_t i = 0; i < nsteps; ++i)
-        {
-            if (!(sweep_flags(w) & (SW_FORCES | SW_MODEL_INPUT)))
-            {
-                if ((rc = step_graph1(w, dt)))
-                    return rc;
-            }
-            else
-            {
-                if ((rc = step_eager(w, dt, false)))
-                    return rc;
-                ++w->eager_steps_run;
-            }
-        }
+            if ((rc = plain_step(w, dt)))
+                return rc;
         return check_status(w);
     }
     rc = ensure_snapshot(w, false);
@@ -1197,25 +1222,12 @@ int plain_steps(nans_world *w, float dt, uint32_t nsteps)
     {
         CK(cudaMemsetAsync(d.cull_max, 0, sizeof(int), st));
         for (uint32_t i = 0; i < nsteps; ++i)
-        {
-            // graphs for the repeating flags (steady steps, and steps after a download or a state
-            // write); the first step after an upload or set_state (forces, input Model) is eager
-            if (!(sweep_flags(w) & (SW_FORCES | SW_MODEL_INPUT)))
-            {
-                if ((rc = step_graph1(w, dt)))
-                    return rc;
-            }
-            else
-            {
-                if ((rc = step_eager(w, dt, false)))
-                    return rc;
-                ++w->eager_steps_run;
-            }
-        }
-        unsigned hdr[2] = {0u, 0u};
-        CK(cudaMemcpyAsync(&hdr[0], d.status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&hdr[1], d.cull_max, sizeof(int), cudaMemcpyDeviceToHost, st));
+            if ((rc = plain_step(w, dt)))
+                return rc;
+        CK(cudaMemcpyAsync(w->h_words, d.status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(w->h_words + 1, d.cull_max, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        const unsigned hdr[2] = {(unsigned)w->h_words[0], (unsigned)w->h_words[1]};
         if (!(hdr[0] & ST_CANDIDATES))
             return status_code(w, hdr[0]);
         // roll back and grow
@@ -1403,6 +1415,8 @@ int nans_world_create(const nans_world_desc *desc, nans_world **out)
     if (e == cudaSuccess)
         e = cudaMallocHost(&w->h_words, 4 * sizeof(int));
     if (e == cudaSuccess)
+        e = cudaMallocHost(&w->h_stage, kHostStage);
+    if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&w->sm_count, cudaDevAttrMultiProcessorCount, w->device);
     if (e == cudaSuccess)
         e = (cudaError_t)narrow_kernel_attrs();
@@ -1422,6 +1436,8 @@ int nans_world_create(const nans_world_desc *desc, nans_world **out)
             cudaEventDestroy(w->ev_pairs);
         if (w->h_words)
             cudaFreeHost(w->h_words);
+        if (w->h_stage)
+            cudaFreeHost(w->h_stage);
         delete w;
         return fail(NANS_ERR_CUDA, std::string("create: ") + cudaGetErrorString(e));
     }
@@ -1451,6 +1467,8 @@ int nans_world_destroy(nans_world *w)
         cudaFree(w->d_tape);
     if (w->h_words)
         cudaFreeHost(w->h_words);
+    if (w->h_stage)
+        cudaFreeHost(w->h_stage);
     if (w->stream)
         cudaStreamDestroy(w->stream);
     if (w->stream2)
@@ -1537,7 +1555,10 @@ int nans_batch_prepare(nans_world *w, float dt, uint32_t graph_steps)
     const uint32_t g = graph_steps ? graph_steps : 60;
     int rc = NANS_OK;
     if (g == 1)
-        rc = ensure_graph1(w, dt);
+    {
+        cudaGraphExec_t exec = nullptr;
+        rc = ensure_graph1(w, dt, &exec);
+    }
     else if (!(sweep_flags(w) & (SW_FORCES | SW_MODEL_INPUT)))
     {
         cudaGraphExec_t exec = nullptr;
@@ -1704,13 +1725,28 @@ int nans_world_download(nans_world *w, nans_cube *cubes, nans_sphere *spheres, n
     k_pack<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(
         w->dw, w->d_rec_cube, w->d_rec_sphere, w->d_rec_floor, w->d_body_rec, w->d_size_moi, w->steps_run > 0);
     CK(cudaGetLastError());
-    if (cubes && w->n_cubes)
-        CK(cudaMemcpyAsync(cubes, w->d_rec_cube, w->n_cubes * sizeof(nans_cube), cudaMemcpyDeviceToHost, st));
-    if (spheres && w->n_spheres)
-        CK(cudaMemcpyAsync(spheres, w->d_rec_sphere, w->n_spheres * sizeof(nans_sphere), cudaMemcpyDeviceToHost, st));
-    if (floors)
-        CK(cudaMemcpyAsync(floors, w->d_rec_floor, w->n_scenes * sizeof(nans_cube), cudaMemcpyDeviceToHost, st));
+    // A copy to pageable memory waits for itself (10 us each); a small world's records come back through
+    // page-locked memory in one wait.
+    void *out[3] = {w->n_cubes ? cubes : nullptr, w->n_spheres ? spheres : nullptr, floors};
+    const float *src[3] = {w->d_rec_cube, w->d_rec_sphere, w->d_rec_floor};
+    const size_t bytes[3] = {w->n_cubes * sizeof(nans_cube), w->n_spheres * sizeof(nans_sphere),
+                             w->n_scenes * sizeof(nans_cube)};
+    const bool staged = bytes[0] + bytes[1] + bytes[2] <= kHostStage;
+    size_t at = 0;
+    for (int i = 0; i < 3; ++i)
+        if (out[i])
+        {
+            CK(cudaMemcpyAsync(staged ? w->h_stage + at : out[i], src[i], bytes[i], cudaMemcpyDeviceToHost, st));
+            at += bytes[i];
+        }
     CK(cudaStreamSynchronize(st));
+    at = 0;
+    for (int i = 0; staged && i < 3; ++i)
+        if (out[i])
+        {
+            std::memcpy(out[i], w->h_stage + at, bytes[i]);
+            at += bytes[i];
+        }
     return NANS_OK;
 }
 
@@ -2013,12 +2049,18 @@ int nans_get_pairs(nans_world *w, uint32_t scene, nans_contact_pair *out, uint32
     }
     k_pairs_out<<<1, 256, 0, st>>>(w->dw, (int)scene, w->d_pairs_out, (int)cap, w->d_small);
     CK(cudaGetLastError());
-    int n = 0;
-    CK(cudaMemcpyAsync(&n, w->d_small, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // a list that fits the page-locked buffer comes back with its count in one wait
+    const bool staged = out && cap && cap * sizeof(nans_contact_pair) <= kHostStage;
+    CK(cudaMemcpyAsync(w->h_words, w->d_small, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (staged)
+        CK(cudaMemcpyAsync(w->h_stage, w->d_pairs_out, cap * sizeof(nans_contact_pair), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    const int n = w->h_words[0];
     *count = (uint32_t)n;
     uint32_t m = std::min<uint32_t>((uint32_t)n, cap);
-    if (out && m)
+    if (staged)
+        std::memcpy(out, w->h_stage, m * sizeof(nans_contact_pair));
+    else if (out && m)
     {
         CK(cudaMemcpyAsync(out, w->d_pairs_out, m * sizeof(nans_contact_pair), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
