@@ -467,6 +467,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     d.n_scenes = S;
     d.n_dyn = ndyn;
     d.solve_cache = solve_cache_bodies(max_bodies);
+    d.solve_rounds = solve_labels_in_rounds(max_bodies) ? 1 : 0;
     d.n_all = nall;
     d.pair_total = pair_acc;
     d.n_words = (int)word_acc;
@@ -749,7 +750,7 @@ cudaError_t enqueue_narrow_solve(nans_world *w, float dt, cudaEvent_t *tl)
     e = (cudaError_t)launch_narrow_big(st2, w->dw);
     if (tl)
         cudaEventRecord(tl[2], st2);
-    launch_solve(w->dw, w->n_scenes, w->solve_threads0 ? w->solve_threads0 : solve_threads(w->max_scene_bodies),
+    launch_solve(w->dw, w->n_scenes, w->solve_threads0 ? w->solve_threads0 : solve_threads(w->max_scene_bodies, w->n_scenes, w->sm_count),
                  solve_smem(w), st, dt, 0);
     if (tl)
         cudaEventRecord(tl[3], st);
@@ -948,7 +949,6 @@ int capture_steps(nans_world *w, float dt, int gsteps, cudaGraphExec_t *exec, fl
     cudaStream_t st = w->stream;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    DevWorld &d = w->dw;
     const bool conditional = use_fused(w) && w->fused_conditional;
     cudaError_t ec = cudaSuccess;
     for (int i = 0; i < gsteps; ++i)
@@ -1622,7 +1622,7 @@ int nans_batch_autotune(nans_world *w, float dt)
     };
     // coordinate descent over the launch parameters, one at a time from the defaults: the cull
     // method (tiles or one lane per pair), the GJK pass's blocks per SM, the solver's threads per
-    // scene in its first pass (1 or 2 warps), its blocks per SM for the late scenes (6 or 2),
+    // scene in its first pass (the default, 1 or 2 warps), its blocks per SM for the late scenes (6 or 2),
     // the warp-tier EPA's blocks per SM (2 or 3) and the late scenes' threads (4 or 2 warps)
     struct Axis
     {
@@ -1630,11 +1630,11 @@ int nans_batch_autotune(nans_world *w, float dt)
         int cands[4];
         int ncand;
     };
-    const int solve0_auto = solve_threads(w->max_scene_bodies);
+    const int solve0_auto = solve_threads(w->max_scene_bodies, w->n_scenes, w->sm_count);
     Axis axes[] = {
         {&w->cull_tiles, {1, 0, 0, 0}, (w->flags & NANS_WORLD_ALL_PAIRS) ? 1 : 2},
         {&w->narrow_bpsm, {0, 4, 0, 0}, 2},
-        {&w->solve_threads0, {solve0_auto, 64, 0, 0}, solve0_auto == 32 ? 2 : 1},
+        {&w->solve_threads0, {solve0_auto, solve0_auto == 64 ? 32 : 64, 0, 0}, w->max_scene_bodies > 512 ? 1 : 2},
         {&w->solve_late_bpsm, {kSolveLateBlocksPerSm, 2, 0, 0}, 2},
         {&w->medium_bpsm, {kMediumBlocksPerSm, 3, 0, 0}, 2},
         {&w->solve_threads1, {kSolveLateThreads, 64, 0, 0}, 2},
@@ -1697,7 +1697,7 @@ int nans_world_tuning(nans_world *w, int32_t *out)
     if (!w || !out)
         return fail(NANS_ERR_INVALID_ARGUMENT, "tuning: null world or output");
     out[0] = w->narrow_bpsm;
-    out[1] = w->solve_threads0 ? w->solve_threads0 : solve_threads(w->max_scene_bodies);
+    out[1] = w->solve_threads0 ? w->solve_threads0 : solve_threads(w->max_scene_bodies, w->n_scenes, w->sm_count);
     out[2] = w->solve_threads1;
     out[3] = w->cull_tiles;
     out[4] = w->solve_late_bpsm;
@@ -2183,7 +2183,6 @@ int nans_profile_steps(nans_world *w, float dt, uint32_t nsteps, float *stage_ms
         CK(cudaEventCreate(&ev[i]));
     for (int i = 0; i < 6; ++i)
         stage_ms[i] = 0.0f;
-    DevWorld &d = w->dw;
     for (uint32_t k = 0; k < nsteps; ++k)
     {
         CK(cudaEventRecord(ev[0], st));
@@ -2197,7 +2196,7 @@ int nans_profile_steps(nans_world *w, float dt, uint32_t nsteps, float *stage_ms
         CK(cudaEventRecord(ev[4], st));
         CK((cudaError_t)launch_narrow_big(st, w->dw));
         CK(cudaEventRecord(ev[5], st));
-        launch_solve(w->dw, w->n_scenes, w->solve_threads0 ? w->solve_threads0 : solve_threads(w->max_scene_bodies),
+        launch_solve(w->dw, w->n_scenes, w->solve_threads0 ? w->solve_threads0 : solve_threads(w->max_scene_bodies, w->n_scenes, w->sm_count),
                  solve_smem(w), st, dt, 0);
         launch_solve(w->dw, std::min(w->n_scenes, w->solve_late_bpsm * w->sm_count), w->solve_threads1, solve_smem(w), st,
                  dt, 1);
@@ -2232,7 +2231,6 @@ int nans_profile_timeline(nans_world *w, float dt, uint32_t nsteps, float *t_ms)
         CK(cudaEventCreate(&ev[i]));
     for (int i = 0; i < 7; ++i)
         t_ms[i] = 0.0f;
-    DevWorld &d = w->dw;
     for (uint32_t k = 0; k < nsteps; ++k)
     {
         CK(cudaEventRecord(ev[0], st));

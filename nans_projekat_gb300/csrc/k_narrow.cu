@@ -1352,7 +1352,7 @@ static_assert(kSceneThreads % 32 == 0 && kSceneThreads <= kWaveChunk, "scene ste
 static_assert((kSceneThreads / 32) * sizeof(WarpEpa) <= 48 * 1024 &&
                   kSceneWarpEpas * sizeof(EpaFast) <= 48 * 1024 &&
                   (size_t)(kSceneStepMaxBodies + 1) * 2 * sizeof(float4) <= 48 * 1024 &&
-                  4 * kWaveChunk * sizeof(int) + kSceneStepMaxBodies * sizeof(int) <= 48 * 1024,
+                  4 * kWaveChunk * sizeof(int) + 2 * kSceneStepMaxBodies * sizeof(int) <= 48 * 1024,
               "scene step shared memory");
 
 size_t scene_step_smem(size_t solve_bytes)

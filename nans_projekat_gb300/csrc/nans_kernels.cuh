@@ -131,7 +131,8 @@ void launch_epa_medium(cudaStream_t st, const DevWorld &w);
 void launch_scene_step(const DevWorld &w, size_t solve_bytes, float dt, int all_pairs, cudaStream_t st,
                        cudaGraphConditionalHandle cond, int signal);
 int tier_priority(); // the device's greatest stream priority
-int solve_threads(int max_scene_bodies);
+int solve_threads(int max_scene_bodies, int n_scenes, int sm_count);
+bool solve_labels_in_rounds(int max_scene_bodies);
 // scenes of up to this many bodies solve on a shared-memory copy of their velocities
 int solve_cache_bodies(int max_scene_bodies);
 // the solver's dynamic shared memory (chunk arrays and per-body waves, or the velocity copy)

@@ -61,10 +61,12 @@ def _compare(batch, steps, step):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n_scenes,lo,hi", [(1, 4, 4), (1, 256, 256), (40, 30, 60), (60, 40, 80)])
+@pytest.mark.parametrize("n_scenes,lo,hi", [(1, 4, 4), (1, 130, 130), (1, 256, 256), (1, 300, 300), (40, 30, 60),
+                                             (60, 40, 80)])
 def test_few_and_many_pairs(oracle_lib, n_scenes, lo, hi):
     """One scene of 4 bodies (10 pairs) up to candidates on both sides of the count (2,432 on a
-    GB300) at which a step leaves the warp-per-pair form, past the impact of the projectile."""
+    GB300) at which a step leaves the warp-per-pair form, past the impact of the projectile; contact
+    lists on both sides of the lengths (128 and 256) at which the solver labels its waves otherwise."""
     from nans_projekat_gb300 import scenes
     batch = scenes.stack_batch(n_scenes, seed=31, lo=lo, hi=hi)
     _compare(batch, 45, lambda w, n: w.step(DT, n))
