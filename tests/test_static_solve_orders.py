@@ -1,7 +1,7 @@
 """nans_solve_contacts_static on contact lists of any order against the oracle's sequential solve
-of the same list, bit for bit: sizes around the block's threads and around the number of bodies
-whose velocities fit shared memory, one body in every contact, repeated contacts of one pair, and the
-entry point's limits."""
+of the same list, bit for bit: sizes around the block's threads, around the length from which a list
+is ordered by a launch of its own, and around the number of bodies whose velocities fit shared
+memory, one body in every contact, repeated contacts of one pair, and the entry point's limits."""
 import numpy as np
 import pytest
 
@@ -47,6 +47,8 @@ def _case(rng, n, m, kind):
 @pytest.mark.parametrize("n,m,kind", [(2, 1, "random"), (3, 7, "random"), (40, 511, "random"), (300, 512, "random"),
                                       (300, 513, "random"), (60, 2000, "star"), (5, 400, "repeated"),
                                       (1500, 1499, "chain"), (6000, 9000, "random"), (6001, 9000, "random"),
+                                      (6001, 500, "random"), (300, 1024, "random"), (300, 1025, "random"),
+                                      (9000, 2500, "random"), (9001, 2500, "random"), (700, 1025, "chain"),
                                       (4913, 16384, "random"), (16384, 16384, "random")])
 def test_solve_equals_the_list_in_order(oracle_lib, n, m, kind):
     import torch
