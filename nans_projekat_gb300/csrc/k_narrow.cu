@@ -967,7 +967,10 @@ __device__ __forceinline__ int gjk_run(const DevWorld &w, int c, int ia, int ib,
     return g;
 }
 
-// Persistent: warps take 32 candidates at a time from a global queue; each lane runs GJK
+// Persistent: warps take 32 candidates at a time, the first batch by the warp's number and the others
+// from a global queue (neighbouring batches, of one scene often and alike in length, start on different
+// SMs, and the first needs no counter: 249 -> 237 us a step's narrowphase for 777 scenes of hulls,
+// 99.5 -> 96 for 1,024 of 33 boxes); each lane runs GJK
 // (budget kGjkShort calls); GJKs that need more calls go to the long pass, so that the rare
 // long GJK runs share warps with each other instead of stalling 31 finished lanes.
 constexpr int kGjkShort = 8;
@@ -978,11 +981,9 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
 {
     const int lane = threadIdx.x & 31;
     const int n = *w.n_cand;
+    const int warps = gridDim.x * (kGjkThreads / 32);
     // the warp claims its next 32 candidates and reads their bodies while it runs these
-    int base = 0;
-    if (lane == 0)
-        base = atomicAdd(w.work_counter, 32);
-    base = __shfl_sync(0xffffffffu, base, 0);
+    int base = 32 * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
     int ia = 0, ib = 0;
     if (base + lane < n)
     {
@@ -993,7 +994,7 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
     {
         int next = 0;
         if (lane == 0)
-            next = atomicAdd(w.work_counter, 32);
+            next = 32 * warps + atomicAdd(w.work_counter, 32);
         next = __shfl_sync(0xffffffffu, next, 0);
         int na = 0, nb = 0;
         if (next + lane < n)
