@@ -130,14 +130,14 @@ __device__ __forceinline__ GV cached_support(const DevWorld &w, const B &E, cons
     else if (A.npts <= B::kShapeCache)
         r.sa = cached_hull_support(E.sva, A.npts, d);
     else
-        r.sa = hull_support(w.verts, A.off, A.npts, d);
+        r.sa = hull_support<true>(w.verts, A.off, A.npts, d);
     const v3 nd = -1.0f * d;
     if (Bs.npts == 0)
         r.sb = sphere_support(Bs.p, Bs.radius, nd);
     else if (Bs.npts <= B::kShapeCache)
         r.sb = cached_hull_support(E.svb, Bs.npts, nd);
     else
-        r.sb = hull_support(w.verts, Bs.off, Bs.npts, nd);
+        r.sb = hull_support<true>(w.verts, Bs.off, Bs.npts, nd);
     r.p = r.sa - r.sb;
     return r;
 }
@@ -683,7 +683,7 @@ __device__ __forceinline__ void load_verts8(const float *verts, int off, Verts8 
 #pragma unroll
     for (int i = 0; i < 6; ++i)
     {
-        const float4 f = __ldg(q + i);
+        const float4 f = q[i];
         v[4 * i] = f.x;
         v[4 * i + 1] = f.y;
         v[4 * i + 2] = f.z;

@@ -46,7 +46,7 @@ __device__ __forceinline__ v3 warp_side(const float *verts, const Shape &s, v3 l
         for (int t = lane; t < s.npts; t += 32)
         {
             const float *p = verts + s.off + 3 * t;
-            const v3 v = mk3(__ldg(p), __ldg(p + 1), __ldg(p + 2));
+            const v3 v = mk3(p[0], p[1], p[2]);
             const float dist = dot3(v, d);
             if (dist > best)
             {
@@ -71,7 +71,7 @@ __device__ __forceinline__ v3 lane_vertex(const float *verts, const Shape &s, in
     if (lane < s.npts && s.npts <= 32)
     {
         const float *p = verts + s.off + 3 * lane;
-        r = mk3(__ldg(p), __ldg(p + 1), __ldg(p + 2));
+        r = mk3(p[0], p[1], p[2]);
     }
     return r;
 }

@@ -156,7 +156,11 @@ struct DevWorld
 // support maps (code/nans.cpp:409-461): argmax of dot(vertex, d) starting at -FLT_MAX with
 // a strict '>' so the first maximum wins and (0,0,0) is returned when nothing beats it.
 // ------------------------------------------------------------------------------------
-__device__ __forceinline__ v3 hull_support(const float *__restrict__ verts, int off, int npts, v3 d)
+// NC: through the read-only path (__ldg). It gave the warp tier 92.5 us against 95 at 16,384 stacks; the
+// GJK, the per-thread EPA and the pair tier read vertices and positions by ordinary loads (237 -> 222 us
+// a step's narrowphase for 777 scenes of hulls, where loops over vertices are most of the reads).
+template <bool NC = false>
+__device__ __forceinline__ v3 hull_support(const float *verts, int off, int npts, v3 d)
 {
     float best = -FLT_MAX;
     v3 r = mk3(0.0f, 0.0f, 0.0f);
@@ -164,7 +168,8 @@ __device__ __forceinline__ v3 hull_support(const float *__restrict__ verts, int 
     int groups = (npts + 3) >> 2;
     for (int g = 0; g < groups; ++g)
     {
-        float4 q0 = __ldg(q + 3 * g), q1 = __ldg(q + 3 * g + 1), q2 = __ldg(q + 3 * g + 2);
+        const float4 q0 = NC ? __ldg(q + 3 * g) : q[3 * g], q1 = NC ? __ldg(q + 3 * g + 1) : q[3 * g + 1],
+                     q2 = NC ? __ldg(q + 3 * g + 2) : q[3 * g + 2];
         v3 v[4] = {mk3(q0.x, q0.y, q0.z), mk3(q0.w, q1.x, q1.y), mk3(q1.z, q1.w, q2.x),
                    mk3(q2.y, q2.z, q2.w)};
 #pragma unroll
@@ -223,7 +228,7 @@ __device__ __forceinline__ bool dev_check(const DevWorld &w, bool ok, int site, 
 __device__ __forceinline__ Shape load_shape(const DevWorld &w, int b)
 {
     Shape s;
-    float4 p = __ldg(w.pos + b);
+    float4 p = w.pos[b];
     int4 sh = __ldg(w.shape + b);
     s.p = mk3(p.x, p.y, p.z);
     s.radius = p.w;
