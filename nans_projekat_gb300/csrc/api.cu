@@ -496,10 +496,10 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
         (rc = dalloc(w, L, &d.epa_hist, (size_t)word_acc * 32)) ||
         (rc = dalloc(w, L, &d.cull_state, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.cull_total, 1)) ||
         (rc = dalloc(w, L, &d.cull_max, 1)) ||
-        (rc = dalloc(w, L, &d.n_cand, 1)) ||
+        (rc = dalloc(w, L, &d.n_cand, 2)) ||
         (rc = dalloc(w, L, &d.cand_begin, S)) || (rc = dalloc(w, L, &d.cand_end, S)) ||
         (rc = dalloc(w, L, &d.scene_late, S)) || (rc = dalloc(w, L, &d.late_list, S)) ||
-        (rc = dalloc(w, L, &d.work_counter, kWorkCounters)) || (rc = dalloc(w, L, &d.status, 1)) ||
+        (rc = dalloc(w, L, &d.work_counter, kWorkCounters)) ||
         (rc = dalloc(w, L, &d.ovf_cand, kEpaOverflowCap)) || (rc = dalloc(w, L, &d.med_cand, kEpaMediumCap)) ||
         (rc = dalloc(w, L, &d.epa_arena, epa_big_bytes())) ||
         (rc = dalloc(w, L, &d.giant_scratch, epa_giant_scratch_bytes())) ||
@@ -510,6 +510,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
         (rc = dalloc(w, L, &w->d_rec_floor, (size_t)61 * S)) || (rc = dalloc(w, L, &w->d_small, 2)) ||
         (rc = dalloc(w, L, &d.s_last, 1)))
         return rc;
+    d.status = reinterpret_cast<unsigned *>(d.n_cand + 1); // beside the count: one copy reads both
     // no EPA seen yet: every pair starts in the short-EPA part of the queue
     CK(cudaMemset(d.epa_hist, 0, std::max(1LL, word_acc * 32)));
     // world vertices are written by the first step; zero until then (the renderer reads them)
@@ -1318,23 +1319,18 @@ int diff_step(nans_world *w, float dt, bool graph)
     int rc;
     if ((rc = tape_alloc(w, &t.v_pre, nd)) || (rc = tape_alloc(w, &t.w_pre, nd)))
         return rc;
-    CK(cudaMemcpyAsync(t.v_pre, d.vel, nd * sizeof(float4), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(t.w_pre, d.omg, nd * sizeof(float4), cudaMemcpyDeviceToDevice, st));
-    if (graph && steady(w, dt))
+    graph = graph && steady(w, dt);
+    const bool may_grow = graph && (long long)w->cand_cap < d.pair_total;
+    if (may_grow && (rc = ensure_snapshot(w, false)))
+        return rc;
+    if (nd)
+        k_tape_pre<<<(int)((nd + 255) / 256), 256, 0, st>>>(d, t, may_grow ? w->d_snap : nullptr);
+    if (graph)
     {
-        const bool may_grow = (long long)w->cand_cap < d.pair_total;
-        if (may_grow)
-        {
-            if ((rc = ensure_snapshot(w, false)))
-                return rc;
-            CK(cudaMemcpyAsync(w->d_snap, d.pos, nd * sizeof(float4), cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(w->d_snap + nd, d.ang, nd * sizeof(float4), cudaMemcpyDeviceToDevice, st));
-        }
         if ((rc = ensure_graph_tape(w, dt)))
             return rc;
         CK(cudaGraphLaunch(w->gexec_t, st));
-        CK(cudaMemcpyAsync(w->h_words, d.n_cand, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(w->h_words + 1, d.status, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(w->h_words, d.n_cand, 2 * sizeof(int), cudaMemcpyDeviceToHost, st)); // and the status
         CK(cudaStreamSynchronize(st));
         if (may_grow && (w->h_words[1] & (int)ST_CANDIDATES))
         {
@@ -1348,8 +1344,6 @@ int diff_step(nans_world *w, float dt, bool graph)
         else
             after_step(w, dt);
     }
-    else
-        graph = false;
     if (!graph)
     {
         if (w->forces_pending)

@@ -150,7 +150,7 @@ __global__ void k_pairs_out(DevWorld w, int scene, float *out_rec, int cap, int 
 struct TapeStep
 {
     int *a, *b, *type;        // per slot: bodies and pair type
-    float4 *k;                // per slot: 9 float4 of contact constants (k_solve layout)
+    float4 *k;                // 9 rows of n float4: the slots' contact constants (k_solve's slot_k)
     float4 *fwd;              // per slot: (JdVn, JdVt1, JdVt2, flags), (dn, dt1, dt2, Ln)
     int *wend;                // per scene, from its first slot: end of each wave (k_solve's s_wcnt)
     int *cand_begin, *maxw;   // per scene
@@ -172,6 +172,7 @@ struct AdjointBufs
 };
 
 int adjoint_threads();
+__global__ void k_tape_pre(DevWorld w, TapeStep t, float4 *snap);
 __global__ void k_tape_copy(DevWorld w, TapeStep t);
 __global__ void k_adjoint(DevWorld w, const TapeStep *steps, int nsteps, float h, AdjointBufs g);
 __global__ void k_rec_to_body(const float *in_rec, const int *body_rec, int n_cubes, int n_dyn, float4 *out);
