@@ -131,13 +131,13 @@ typedef struct nans_contact_pair
                                       32 pairs per warp (faster on the benchmark workload).
                                       Results are the same. */
 #define NANS_WORLD_FUSED_STEP 64u  /* one launch per step detects and solves each scene (cull,
-                                      GJK, EPA on the per-thread and warp tiers, solve; a block
+                                      GJK, EPA on the pair and warp tiers, solve; a block
                                       per scene) after the sweep, in place of the staged
                                       kernels; EPAs beyond the warp tier still take the large
                                       tiers and the late solve pass. Same results. For worlds of a
                                       few small scenes, where the staged step's launch chain is
                                       the cost (the reference's own scene); a world with a scene of
-                                      more than 24 bodies or more scenes than the GPU has SMs takes
+                                      more than 12 bodies or more scenes than the GPU has SMs takes
                                       the staged kernels, which are faster there. Scenes of at most 1,024
                                       bodies; the candidate buffers hold every pair (the
                                       max_candidates request is raised to that); not with
@@ -257,8 +257,8 @@ int nans_world_counts(nans_world *world, uint32_t *candidates, uint32_t *contact
 /* Large-polytope EPA statistics since upload (or the last reset): out[0] largest face list
  * and out[1] largest horizon seen by the block and giant tiers, out[2] EPAs that went beyond
  * the warp tier, out[3] candidate index + 1 and out[4] scene + 1 of the last EPA that outgrew
- * the giant tier (0 if none), out[5] EPAs that outgrew it, out[6] EPAs escalated from the
- * per-thread tier to the warp tier, out[7] EPAs escalated from the block tier (32,768 faces)
+ * the giant tier (0 if none), out[5] EPAs that outgrew it, out[6] EPAs escalated to the
+ * warp tier, out[7] EPAs escalated from the block tier (32,768 faces)
  * to the giant tier. out holds 8 entries. */
 int nans_world_epa_stats(nans_world *world, uint32_t *out, int reset);
 
@@ -270,7 +270,7 @@ void *nans_world_stream(nans_world *world);
  * (code/sdl_nans.cpp:994-1005).
  * Runs nsteps steps stage by stage with CUDA events on the world's stream between the
  * stages and adds each stage's device time in milliseconds to stage_ms[0..5]:
- * [0] integrate sweep, [1] pair cull (3 kernels), [2] narrowphase (GJK + per-thread EPA),
+ * [0] integrate sweep, [1] pair cull, [2] narrowphase (GJK, per-thread EPA, pair tier),
  * [3] warp-tier EPA, [4] large-polytope EPA, [5] solver. */
 int nans_profile_steps(nans_world *world, float dt, uint32_t nsteps, float *stage_ms);
 

@@ -2,11 +2,12 @@
 //
 // A world owns one CUDA stream and every device buffer of its scenes. The step is the
 // stage sequence of the reference's frame function (code/nans.cpp:1758-1762) plus the
-// render code's Model rebuild, as six kernels:
-//   k_sweep        IntegrateVelocities(prev) + rebuild + IntegrateForces + vertices + AABB
-//   k_cull_mask / k_cull_scan / k_cull_write     ordered candidate pairs
-//   k_narrow / k_narrow_big   GJK + EPA           (DetectCollisions)
-//   k_solve        sequential impulses by waves   (SolveConstraints)
+// render code's Model rebuild:
+//   k_sweep                       IntegrateVelocities(prev) + rebuild + IntegrateForces + vertices + AABB
+//   k_cull_tiles / k_cull_place   ordered candidate pairs
+//   k_gjk / k_epa_tiny / k_pair_warp / k_epa_medium / k_epa_block / k_epa_giant
+//                                 GJK + EPA           (DetectCollisions)
+//   k_solve                       sequential impulses by waves   (SolveConstraints)
 // The last step's IntegrateVelocities is folded into the next step's sweep, or applied by
 // nans_world_download.
 #include <cuda_runtime.h>
@@ -548,9 +549,11 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     d.medium_blocks = std::min(w->medium_bpsm * w->sm_count, w->medium_cap_blocks);
     d.tiny_blocks = upto(64, epa_tiny_grid(w->sm_count));
     d.pair_blocks = upto(2, pair_warp_grid(w->sm_count));
-    // The fused step runs a scene on one block, so it pays while a scene's pairs fit the block's warps
-    // and every scene has an SM: 57.7 against 73.6 us a step for one scene of 9 bodies and 58.0 against
-    // 69.4 for 16, but 103 against 90 for 32 and 377 against 114 for 256.
+    // The fused step runs a scene on one block, so it pays while a scene's pairs go through the block's
+    // warps in a few turns and every scene has an SM. Fused and staged, us a step of a call of 40 steps:
+    // one scene of 4 bodies 43 and 50, of 9 58 and 57, of 16 58 and 53, of 24 60 and 54; 30 scenes of 4
+    // 73 and 78, of 12 78 and 74, of 24 97 and 84; 150 scenes of 4 75 and 84, of 12 88 and 94, of 24 108
+    // and 106. One step a call: 52 and 63 at 4 bodies, 65 and 66 at 9, 70 and 64 at 24.
     w->fused_small = w->fused && max_bodies <= kSceneStepBodies && S <= w->sm_count;
     // Steps of up to 16 candidates per SM give each pair a warp from the start of its GJK (136 against
     // 142 us a step at 2,000 candidates; 197 against 162 at 6,400: then a thread per pair).

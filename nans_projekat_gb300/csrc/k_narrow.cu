@@ -1333,7 +1333,7 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32) k_epa_medium(
 // block of kSceneThreads threads takes a scene at a time (largest first) and runs its whole
 // detect-and-solve sequence, each phase on the block:
 //   (1) the cull: the scene's pairs in the reference's order (code/nans.cpp:1355-1535), kept
-//       when their inflated boxes meet (k_cull_mask's test), compacted in order by block scans
+//       when their inflated boxes meet (k_cull_place's test), compacted in order by block scans
 //       into the scene's own slots of the pair space (from sc_word0 * 32: the candidate
 //       buffers of such a world hold every pair, so no scan across scenes is needed);
 //   (2) GJK and EPA, a warp per candidate (pair_warp);

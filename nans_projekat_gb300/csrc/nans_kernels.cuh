@@ -41,18 +41,19 @@ constexpr int kWaveChunk = 256;     // solver: candidates compacted and labelled
 constexpr size_t kSolveSmemMax = 200 * 1024; // solver: dynamic shared memory per block, at most
 constexpr int kMediumBlocksPerSm = 2;    // warp-tier EPA blocks per SM (shared memory allows three)
 constexpr int kSceneStepMaxBodies = 1024; // fused per-scene worlds: bodies per scene, at most
-constexpr int kSceneStepBodies = 24;     // fused per-scene step: larger scenes take the staged kernels
+constexpr int kSceneStepBodies = 12;     // fused per-scene step: larger scenes take the staged kernels
 
 // EPA capacities. Vertices: the GJK tetrahedron plus one support per EPA iteration (at most
 // 65, code/nans.cpp:804). Faces grow by two per iteration on a convex polytope, but the
 // reference's polytope is not always convex: with bodies flung to large coordinates the
 // supports repeat existing vertices, faces degenerate (NaN normals, never removed) and the
 // list keeps growing, at times geometrically, for all 65 iterations. On the 16,384-scene
-// stack workload ~1.3 EPAs in a thousand outgrow 12 vertices / 20 faces, ~14 in a million
+// stack workload ~1 EPA in a thousand outgrows 34 vertices / 64 faces, ~14 in a million
 // exceed 128 faces (nearly all of them stay within 256), and the largest met so far (scene
 // 10198, step 135) reaches 485,688 faces and a 139,111-edge horizon (the reference's own
-// algorithm needs 334 s of one CPU core for it). Tier 1 runs EPA per thread (12 vertices, 20
-// faces, 12 edges); tier 2 per warp in shared memory (256 faces, a 64-edge horizon); tier 3
+// algorithm needs 334 s of one CPU core for it). Tier 1 runs EPA per thread (11 vertices, 16
+// faces, 8 edges), and what outgrows it per warp in registers (the pair tier: 34 vertices, 64 faces, 32
+// edges); tier 2 per warp in shared memory (256 faces, a 64-edge horizon); tier 3
 // per block in a global-memory arena of 32,768 faces, two blocks per SM; tier 4 on the whole
 // grid (cooperative launch) in an arena of 8,388,608 faces and 4,194,304 horizon edges.
 // Beyond that the pair gets no contact and the event is counted (NANS_ERR_EPA_CAPACITY in
