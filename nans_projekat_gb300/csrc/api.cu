@@ -496,8 +496,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
         (rc = dalloc(w, L, &p_tiles, tiles.size())) || (rc = dalloc(w, L, &p_rest, rest_tasks.size())) ||
         (rc = dalloc(w, L, &d.epa_hist, (size_t)word_acc * 32)) ||
         (rc = dalloc(w, L, &d.cull_state, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.cull_total, 1)) ||
-        (rc = dalloc(w, L, &d.cull_max, 1)) ||
-        (rc = dalloc(w, L, &d.n_cand, 2)) ||
+        (rc = dalloc(w, L, &d.n_cand, 3)) ||
         (rc = dalloc(w, L, &d.cand_begin, S)) || (rc = dalloc(w, L, &d.cand_end, S)) ||
         (rc = dalloc(w, L, &d.scene_late, S)) || (rc = dalloc(w, L, &d.late_list, S)) ||
         (rc = dalloc(w, L, &d.work_counter, kWorkCounters)) ||
@@ -511,7 +510,8 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
         (rc = dalloc(w, L, &w->d_rec_floor, (size_t)61 * S)) || (rc = dalloc(w, L, &w->d_small, 2)) ||
         (rc = dalloc(w, L, &d.s_last, 1)))
         return rc;
-    d.status = reinterpret_cast<unsigned *>(d.n_cand + 1); // beside the count: one copy reads both
+    d.status = reinterpret_cast<unsigned *>(d.n_cand + 1); // side by side: one copy reads them
+    d.cull_max = d.n_cand + 2;
     // no EPA seen yet: every pair starts in the short-EPA part of the queue
     CK(cudaMemset(d.epa_hist, 0, std::max(1LL, word_acc * 32)));
     // world vertices are written by the first step; zero until then (the renderer reads them)
@@ -1215,9 +1215,8 @@ int plain_steps(nans_world *w, float dt, uint32_t nsteps)
     rc = ensure_snapshot(w, false);
     if (rc)
         return rc;
-    float4 *bufs[6] = {d.pos, d.ang, d.vel, d.omg, d.frc, d.trq};
-    for (int i = 0; i < 6; ++i)
-        CK(cudaMemcpyAsync(w->d_snap + i * n, bufs[i], n * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+    const int grid = (int)((n + 255) / 256);
+    k_state_aside<<<grid, 256, 0, st>>>(d, w->d_snap, (int)n, 0);
     const bool s_pending = w->pending, s_model = w->model_input, s_forces = w->forces_pending;
     const float s_pdt = w->pending_dt;
     const long long s_steps = w->steps_run;
@@ -1228,15 +1227,13 @@ int plain_steps(nans_world *w, float dt, uint32_t nsteps)
         for (uint32_t i = 0; i < nsteps; ++i)
             if ((rc = plain_step(w, dt)))
                 return rc;
-        CK(cudaMemcpyAsync(w->h_words, d.status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(w->h_words + 1, d.cull_max, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(w->h_words, d.status, 2 * sizeof(int), cudaMemcpyDeviceToHost, st)); // and cull_max
         CK(cudaStreamSynchronize(st));
         const unsigned hdr[2] = {(unsigned)w->h_words[0], (unsigned)w->h_words[1]};
         if (!(hdr[0] & ST_CANDIDATES))
             return status_code(w, hdr[0]);
         // roll back and grow
-        for (int i = 0; i < 6; ++i)
-            CK(cudaMemcpyAsync(bufs[i], w->d_snap + i * n, n * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+        k_state_aside<<<grid, 256, 0, st>>>(d, w->d_snap, (int)n, 1);
         w->pending = s_pending;
         w->model_input = s_model;
         w->forces_pending = s_forces;
@@ -1712,30 +1709,32 @@ int nans_world_download(nans_world *w, nans_cube *cubes, nans_sphere *spheres, n
         return fail(NANS_ERR_NOT_UPLOADED, "download: no scene uploaded");
     CK(cudaSetDevice(w->device));
     cudaStream_t st = w->stream;
-    if (w->pending)
-    {
-        k_sweep<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(w->dw, w->pending_dt, 0.0f,
-                                                                                           SW_APPLY_VEL);
-        w->pending = false;
-        w->model_input = false;
-    }
-    k_pack<<<(w->n_all + kSweepThreads - 1) / kSweepThreads, kSweepThreads, 0, st>>>(
-        w->dw, w->d_rec_cube, w->d_rec_sphere, w->d_rec_floor, w->d_body_rec, w->d_size_moi, w->steps_run > 0);
-    CK(cudaGetLastError());
-    // A copy to pageable memory waits for itself (10 us each); a small world's records come back through
-    // page-locked memory in one wait.
+    // A copy to pageable memory waits for itself (10 us each); a small world's records are packed into
+    // page-locked memory, without a copy.
     void *out[3] = {w->n_cubes ? cubes : nullptr, w->n_spheres ? spheres : nullptr, floors};
     const float *src[3] = {w->d_rec_cube, w->d_rec_sphere, w->d_rec_floor};
     const size_t bytes[3] = {w->n_cubes * sizeof(nans_cube), w->n_spheres * sizeof(nans_sphere),
                              w->n_scenes * sizeof(nans_cube)};
     const bool staged = bytes[0] + bytes[1] + bytes[2] <= kHostStage;
+    float *pack[3] = {w->d_rec_cube, w->d_rec_sphere, nullptr};
     size_t at = 0;
-    for (int i = 0; i < 3; ++i)
+    for (int i = 0; staged && i < 3; ++i)
+    {
+        pack[i] = out[i] ? (float *)(w->h_stage + at) : nullptr;
+        at += out[i] ? bytes[i] : 0;
+    }
+    k_pack<<<(w->n_all + kPackThreads - 1) / kPackThreads, kPackThreads, 0, st>>>(
+        w->dw, w->pending_dt, w->pending, pack[0], pack[1], w->d_rec_floor, pack[2], w->d_body_rec, w->d_size_moi,
+        w->steps_run > 0);
+    CK(cudaGetLastError());
+    if (w->pending)
+    {
+        w->pending = false;
+        w->model_input = false;
+    }
+    for (int i = 0; !staged && i < 3; ++i)
         if (out[i])
-        {
-            CK(cudaMemcpyAsync(staged ? w->h_stage + at : out[i], src[i], bytes[i], cudaMemcpyDeviceToHost, st));
-            at += bytes[i];
-        }
+            CK(cudaMemcpyAsync(out[i], src[i], bytes[i], cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     at = 0;
     for (int i = 0; staged && i < 3; ++i)
@@ -2044,13 +2043,10 @@ int nans_get_pairs(nans_world *w, uint32_t scene, nans_contact_pair *out, uint32
         CK(cudaMalloc(&w->d_pairs_out, (size_t)std::max<uint32_t>(cap, 1) * sizeof(nans_contact_pair)));
         w->pairs_out_cap = (int)std::max<uint32_t>(cap, 1);
     }
-    k_pairs_out<<<1, 256, 0, st>>>(w->dw, (int)scene, w->d_pairs_out, (int)cap, w->d_small);
-    CK(cudaGetLastError());
-    // a list that fits the page-locked buffer comes back with its count in one wait
+    // the count, and a list that fits the page-locked buffer, are written there without a copy
     const bool staged = out && cap && cap * sizeof(nans_contact_pair) <= kHostStage;
-    CK(cudaMemcpyAsync(w->h_words, w->d_small, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if (staged)
-        CK(cudaMemcpyAsync(w->h_stage, w->d_pairs_out, cap * sizeof(nans_contact_pair), cudaMemcpyDeviceToHost, st));
+    k_pairs_out<<<1, 256, 0, st>>>(w->dw, (int)scene, staged ? (float *)w->h_stage : w->d_pairs_out, (int)cap, w->h_words);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(st));
     const int n = w->h_words[0];
     *count = (uint32_t)n;

@@ -86,10 +86,12 @@ template <bool WARM> __global__ void __launch_bounds__(kSolveThreadsMax) k_solve
 }
 
 // Writes the contact list of one scene in the reference record layout (code/nans.h:338-372),
-// in list order. Single block.
-__global__ void k_pairs_out(DevWorld w, int scene, float *out_rec, int cap, int *count)
+// in list order. Single block; the records go out as consecutive words, also to page-locked host memory.
+constexpr int kPairsOutThreads = 256;
+__global__ void __launch_bounds__(kPairsOutThreads) k_pairs_out(DevWorld w, int scene, float *out_rec, int cap, int *count)
 {
     __shared__ int sh[32];
+    __shared__ float s_rec[kPairsOutThreads][25];
     const int cb = w.cand_begin[scene], ce = w.cand_end[scene];
     const int c0 = w.sc_cube0[scene], s0 = c0 + w.sc_nc[scene];
     int n = 0;
@@ -106,7 +108,7 @@ __global__ void k_pairs_out(DevWorld w, int scene, float *out_rec, int cap, int 
             int a = w.cand_a[i], b = w.cand_b[i];
             int ia = type_a_is_sphere(type) ? a - s0 : a - c0;
             int ib = type_b_is_floor(type) ? ia : (type_b_is_sphere(type) ? b - s0 : b - c0);
-            float *r = out_rec + (size_t)slot * 24;
+            float *r = s_rec[pre];
             int *ri = reinterpret_cast<int *>(r);
             for (int q = 0; q < 24; ++q)
                 r[q] = 0.0f;
@@ -124,6 +126,11 @@ __global__ void k_pairs_out(DevWorld w, int scene, float *out_rec, int cap, int 
             ri[22] = ia;
             ri[23] = ib;
         }
+        __syncthreads();
+        const int words = 24 * max(0, min(tot, cap - n));
+        for (int k = threadIdx.x; k < words; k += blockDim.x)
+            out_rec[(size_t)n * 24 + k] = s_rec[k / 24][k % 24];
+        __syncthreads(); // the records' memory is the next round's
         n += tot;
     }
     if (threadIdx.x == 0)

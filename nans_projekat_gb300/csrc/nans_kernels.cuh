@@ -91,8 +91,10 @@ constexpr int kEpaMediumCap = 1 << 20; // tier-2 EPAs queued per step
 __global__ void k_sweep(DevWorld w, float pending_dt, float dt, int flags);
 __global__ void k_unpack(DevWorld w, const float *rec_cube, const float *rec_sphere, const float *rec_floor,
                          const int *body_rec, int mode, float4 *prm_out, float4 *model_out);
-__global__ void k_pack(DevWorld w, float *rec_cube, float *rec_sphere, float *rec_floor, const int *body_rec,
-                       const float2 *size_moi, int vertices_valid);
+constexpr int kPackThreads = 64;
+__global__ void k_pack(DevWorld w, float dt, int apply, float *rec_cube, float *rec_sphere, float *rec_floor,
+                       float *floor_out, const int *body_rec, const float2 *size_moi, int vertices_valid);
+__global__ void k_state_aside(DevWorld w, float4 *snap, int n, int back);
 
 __global__ void k_sincos(const float *x, float *s, float *c, int n);
 __global__ void k_state_in(DevWorld w, const float *stage, const int *body_rec, int n_cubes, int mask);
