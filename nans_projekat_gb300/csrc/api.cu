@@ -2001,27 +2001,30 @@ int nans_world_get_state_arrays(nans_world *w, float *position, float *angles, f
     if (!w->d_state_stage && (rc = dalloc(w, w->allocs, &w->d_state_stage, 4 * n3)))
         return rc;
     const int nb = (w->n_all + kSweepThreads - 1) / kSweepThreads;
-    if (w->pending)
-    {
-        k_sweep<<<nb, kSweepThreads, 0, st>>>(w->dw, w->pending_dt, 0.0f, SW_APPLY_VEL);
-        w->pending = false;
-        w->model_input = false;
-    }
     float *dst[4] = {position, angles, velocity, omega};
     int mask = 0;
     for (int q = 0; q < 4; ++q)
         if (dst[q])
             mask |= 1 << q;
-    if (mask && n3)
-    {
-        k_state_out<<<nb, kSweepThreads, 0, st>>>(w->dw, w->d_state_stage, w->d_body_rec, w->n_cubes, mask);
-        for (int q = 0; q < 4; ++q)
-            if (dst[q])
-                CK(cudaMemcpyAsync(dst[q], w->d_state_stage + q * n3, n3 * sizeof(float), cudaMemcpyDeviceToHost,
-                                   st));
-    }
+    // a small world's arrays are written to page-locked memory by the kernel, without a copy
+    const bool staged = 4 * n3 * sizeof(float) <= kHostStage;
+    if ((mask || w->pending) && n3)
+        k_state_out<<<nb, kSweepThreads, 0, st>>>(w->dw, w->pending_dt, w->pending,
+                                                  staged ? (float *)w->h_stage : w->d_state_stage, w->d_body_rec,
+                                                  w->n_cubes, mask);
     CK(cudaGetLastError());
+    if (w->pending)
+    {
+        w->pending = false;
+        w->model_input = false;
+    }
+    for (int q = 0; !staged && n3 && q < 4; ++q)
+        if (dst[q])
+            CK(cudaMemcpyAsync(dst[q], w->d_state_stage + q * n3, n3 * sizeof(float), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    for (int q = 0; staged && n3 && q < 4; ++q)
+        if (dst[q])
+            std::memcpy(dst[q], w->h_stage + q * n3 * sizeof(float), n3 * sizeof(float));
     return NANS_OK;
 }
 

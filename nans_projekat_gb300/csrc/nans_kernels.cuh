@@ -98,7 +98,7 @@ __global__ void k_state_aside(DevWorld w, float4 *snap, int n, int back);
 
 __global__ void k_sincos(const float *x, float *s, float *c, int n);
 __global__ void k_state_in(DevWorld w, const float *stage, const int *body_rec, int n_cubes, int mask);
-__global__ void k_state_out(DevWorld w, float *stage, const int *body_rec, int n_cubes, int mask);
+__global__ void k_state_out(DevWorld w, float dt, int apply, float *stage, const int *body_rec, int n_cubes, int mask);
 
 __global__ void k_cull_tiles(DevWorld w);
 // mask: the blocks make their mask words themselves
