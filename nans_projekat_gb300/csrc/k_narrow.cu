@@ -976,7 +976,8 @@ __device__ __forceinline__ int gjk_run(const DevWorld &w, int c, int ia, int ib,
 constexpr int kGjkShort = 8;
 constexpr int kGjkThreads = 128;
 // four blocks per SM (at most 128 registers, room for both shapes' vertices): measured best
-// against 5 and 6 (which spill the vertices) on the stack workload
+// against 5 and 6 (which spill the vertices) on the stack workload. Bound by issue (0.5 a cycle and
+// scheduler) and by the chain of loads before a batch (half of the stalls); 146 us a step of 16,384 stacks.
 __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
 {
     const int lane = threadIdx.x & 31;
@@ -1178,7 +1179,8 @@ __global__ void __launch_bounds__(kGjkWarpThreads) k_gjk_warp(DevWorld w)
 }
 
 // Tier 1 EPA: one thread per hit from the queue; the polytopes it does not hold go to the pair
-// tier.
+// tier. Bound by issue: 0.63 instructions a cycle and scheduler at 15.6 of 32 lanes, eight blocks of
+// 64 threads per SM by registers (128) and by shared memory alike; 270 us a step of 16,384 stacks.
 __global__ void __launch_bounds__(kTinyThreads, 8) k_epa_tiny(DevWorld w)
 {
     __shared__ TinySmem S;
@@ -1255,7 +1257,9 @@ __device__ __forceinline__ int pair_warp(const DevWorld &w, WarpEpa &S, int c, b
 // The pair tier: a warp per queued pair first finishes its GJK where the first pass left it (hulls
 // of more than eight points, runs of more than kGjkShort calls), then runs its EPA. EPAs that
 // outgrow the warp's registers are queued for the warp tier. Warps stride over the queue. `part`
-// names the entries: the queue's front or back, or every candidate from the start of its GJK.
+// names the entries: the queue's front or back, or every candidate from the start of its GJK. Bound by
+// one pair's chain of dependent calls and iterations, in a small world also by its code's first
+// fetch; ten blocks of two warps per SM by registers (14 and 16 gave nothing).
 __global__ void __launch_bounds__(kPairThreads, 10) k_pair_warp(DevWorld w, int part)
 {
     __shared__ WarpEpa sm[kPairThreads / 32];
