@@ -36,6 +36,8 @@ constexpr int kSolveThreadsMax = 256;
 // pass 0 solves every scene whose contacts are all known after the per-thread EPA tier
 // (largest first, a block per scene); pass 1 the scenes with a candidate in the later EPA
 // tiers (a persistent grid over the late list), so that pass 0 can run while those tiers do.
+// Bound by latency: the round trips to the contacts' geometry in the placement, then a chain of waves
+// (0.39 instructions a cycle and scheduler, 16 warps an SM by registers; 178 us a step of 16,384 stacks).
 template <bool WARM> __global__ void __launch_bounds__(kSolveThreadsMax) k_solve(DevWorld w, float dt, int pass)
 {
     extern __shared__ float4 s_dyn[];
