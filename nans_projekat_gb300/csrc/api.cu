@@ -82,7 +82,7 @@ struct nans_world
     float *d_rec_cube = nullptr, *d_rec_sphere = nullptr, *d_rec_floor = nullptr;
     float *d_pairs_out = nullptr;
     int pairs_out_cap = 0;
-    int *h_words = nullptr; // page-locked: status word, counts read back after a step
+    int *h_words = nullptr; // page-locked: status word, counts read back after a step; [2] a status to set
     unsigned char *h_stage = nullptr; // page-locked, kHostStage bytes: small downloads in one wait
     int *d_small = nullptr; // [0] pair count for k_pairs_out, [1] contact count
     float4 *d_snap = nullptr;
@@ -137,6 +137,7 @@ struct nans_world
     bool fused_small = false;       // its scenes are few and small enough to step faster that way
     bool fused_conditional = true;  // its graphs put the large tiers in a conditional node
     bool tape_valid = false;        // the tape describes the rollout that led to the state
+    unsigned tape_status = 0;       // status bits of the rollout's steps so far
     float tape_dt = 0.0f;
     float4 *fwd_buf = nullptr;      // 2 float4 per candidate slot (in cand_allocs)
     int *d_maxw = nullptr;          // per scene (in allocs)
@@ -868,6 +869,14 @@ cudaError_t enqueue_fused_conditional(nans_world *w, float pending_dt, float dt,
     return et != cudaSuccess ? et : e;
 }
 
+// Sets the status word on the world's stream; a page-locked word of the world carries it.
+int set_status(nans_world *w, unsigned status)
+{
+    w->h_words[2] = (int)status;
+    CK(cudaMemcpyAsync(w->dw.status, w->h_words + 2, sizeof(unsigned), cudaMemcpyHostToDevice, w->stream));
+    return NANS_OK;
+}
+
 // One step, stage by stage. With check_capacity the candidate count is read back after the
 // scan and the candidate buffers grow if needed (the plain path).
 int step_eager(nans_world *w, float dt, bool check_capacity)
@@ -885,9 +894,9 @@ int step_eager(nans_world *w, float dt, bool check_capacity)
     CK(cudaGetLastError());
     if (check_capacity)
     {
-        unsigned status = 0;
-        CK(cudaMemcpyAsync(&status, d.status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(w->h_words, d.status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        const unsigned status = (unsigned)w->h_words[0];
         if (status & ST_CANDIDATES)
         {
             // the scan recorded the exact total: grow the candidate buffers and write again
@@ -897,7 +906,8 @@ int step_eager(nans_world *w, float dt, bool check_capacity)
             int rc = alloc_candidates(w, (int)std::min<long long>((long long)total + total / 4 + 1024, INT32_MAX / 16));
             if (rc)
                 return rc;
-            CK(cudaMemsetAsync(d.status, 0, sizeof(unsigned), st));
+            if ((rc = set_status(w, status & ~(unsigned)ST_CANDIDATES))) // the call's earlier steps' bits stay
+                return rc;
             // what the sweep cleared for the first try
             CK(cudaMemsetAsync(d.work_counter, 0, kWorkCounters * sizeof(int), st));
             CK(cudaMemsetAsync(d.cull_state, 0, w->cull_blocks * sizeof(unsigned long long), st));
@@ -1338,7 +1348,8 @@ int diff_step(nans_world *w, float dt, bool graph)
             CK(cudaMemcpyAsync(d.ang, w->d_snap + nd, nd * sizeof(float4), cudaMemcpyDeviceToDevice, st));
             CK(cudaMemcpyAsync(d.vel, t.v_pre, nd * sizeof(float4), cudaMemcpyDeviceToDevice, st));
             CK(cudaMemcpyAsync(d.omg, t.w_pre, nd * sizeof(float4), cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemsetAsync(d.status, 0, sizeof(unsigned), st));
+            if ((rc = set_status(w, w->tape_status)))
+                return rc;
             graph = false;
         }
         else
@@ -1355,9 +1366,10 @@ int diff_step(nans_world *w, float dt, bool graph)
         }
         if ((rc = step_eager(w, dt, true)))
             return rc;
-        CK(cudaMemcpyAsync(w->h_words, d.n_cand, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(w->h_words, d.n_cand, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
     }
+    w->tape_status = (unsigned)w->h_words[1];
     const int nc = std::max(0, std::min(w->h_words[0], w->cand_cap));
     if ((rc = tape_alloc(w, &t.a, nc)) || (rc = tape_alloc(w, &t.b, nc)) || (rc = tape_alloc(w, &t.type, nc)) ||
         (rc = tape_alloc(w, &t.k, (size_t)9 * nc)) || (rc = tape_alloc(w, &t.fwd, (size_t)2 * nc)) ||
@@ -1796,6 +1808,7 @@ int nans_diff_forward(nans_world *w, const nans_step_params *params, float dt, u
     w->tape_chunk = 0;
     w->tape_off = 0;
     w->tape_bytes = 0;
+    w->tape_status = 0;
     w->tape_valid = false;
     int rc = NANS_OK;
     if (!w->d_maxw && (rc = dalloc(w, w->allocs, &w->d_maxw, w->n_scenes)))
