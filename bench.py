@@ -395,7 +395,7 @@ def schedule_ab(lib, batch, device, warm=25, n=10):
 
 
 def fused_ab(lib, batch, device, warm=5, n=20):
-    """The staged step (10 to 14 kernels, each over the whole world) against the fused step
+    """The staged step (8 to 13 kernels, each over the whole world) against the fused step
     (NANS_WORLD_FUSED_STEP: after the sweep, one launch in which a block per scene culls, collides
     and solves) on identical windows: each world steps the same scenes from the upload (the
     results are the same bit for bit), then n steps from one CUDA graph are timed with CUDA

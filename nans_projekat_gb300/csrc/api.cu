@@ -2278,12 +2278,13 @@ int nans_launches_per_step(nans_world *w, uint32_t *batched, uint32_t *plain)
 {
     if (!w)
         return fail(NANS_ERR_INVALID_ARGUMENT, "launches: null world");
-    // sweep, [cull mask, cull write], cull scan, the narrowphase (the pair tier alone, or GJK,
-    // [its long runs], the pair tier's front, the per-thread EPA, the pair tier's back), epa_medium,
-    // block EPA, giant EPA, solve (two passes); fused: sweep, scene step, block EPA, giant EPA,
-    // late solve
+    // sweep; the cull's tiles and placement, or the placement alone; the narrowphase (the pair tier
+    // alone, or GJK, [its long runs], the pair tier's front, the per-thread EPA, the pair tier's back);
+    // epa_medium, block EPA, giant EPA, solve (two passes). Fused: sweep, scene step, block EPA, giant
+    // EPA, late solve.
+    const uint32_t cull = w->cull_blocks <= 0 ? 0u : (cull_by_lane(w) ? 1u : 2u);
     const uint32_t narrow = w->pair_only ? 1u : (w->long_gjk ? 5u : 4u);
-    uint32_t k = w->fused_small ? 5u : 7 + narrow + (w->cull_blocks > 0 ? 2u : 0u);
+    const uint32_t k = w->fused_small ? 5u : 6u + cull + narrow;
     if (batched)
         *batched = k;
     if (plain)
