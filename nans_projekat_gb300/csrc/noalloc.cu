@@ -709,14 +709,28 @@ extern "C" int nans_solve_contacts_static(uint32_t nbodies, uint32_t ncubes, con
             e = cudaGetSymbolAddress(&p, g_solve_scratch);
             if (e != cudaSuccess || !p)
                 return static_fail(NANS_ERR_CUDA, "nans_solve_contacts_static: cudaGetSymbolAddress failed");
-            // the kernel's shared memory limit, which belongs to the device's context as well
-            const void *kernels[] = {(const void *)k_solve_static, (const void *)k_static_order,
-                                     (const void *)k_static_waves};
-            for (const void *k : kernels)
+            // Every kernel is loaded here (kernels load lazily, and one's code takes device memory), and
+            // those with large dynamic shared memory get their limit, which belongs to the device's
+            // context as well.
+            const struct
+            {
+                const void *fn;
+                bool large;
+            } kernels[] = {{(const void *)k_solve_static, true},
+                           {(const void *)k_static_decode, false},
+                           {(const void *)k_static_order, true},
+                           {(const void *)k_static_constants, false},
+                           {(const void *)k_static_waves, true}};
+            for (const auto &k : kernels)
+            {
+                cudaFuncAttributes attr;
                 if (e == cudaSuccess)
-                    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynamicMax);
+                    e = cudaFuncGetAttributes(&attr, k.fn);
+                if (e == cudaSuccess && k.large)
+                    e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynamicMax);
+            }
             if (e != cudaSuccess)
-                return static_fail(NANS_ERR_CUDA, "nans_solve_contacts_static: shared memory limit");
+                return static_fail(NANS_ERR_CUDA, "nans_solve_contacts_static: kernel set-up");
             g_scratch_addr[dev].ptr = p;
             g_scratch_addr[dev].ctx = ctx;
         }
