@@ -527,8 +527,36 @@ __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, 
     // (4) placement in wave order with the velocity-independent constants: slot cb + pos
     // gets the contact's ids and constants. The slots are the scene's own candidate slots
     // (nh <= ce - cb), whose narrowphase use (the simplex of a hit) ended with the per-thread
-    // EPA; the order of the contacts inside a wave is immaterial (they commute exactly). A
+    // EPA; the order of the contacts inside a wave is immaterial to the solve (they commute exactly). A
     // scene of one chunk takes its hits from shared memory, a larger one from s_order.
+    //
+    // On a tape the order matters to rounding: the adjoint sums the gradients of restitution and friction
+    // over the slots. There a wave's contacts keep list order, so that the same rollout gives the same
+    // gradients: one warp turns the waves into places 32 hits at a time (the atomics alone give the order of
+    // a block's warps; a block of one warp has but one).
+    const bool ordered = !WARM && w.s_fwd != nullptr && blockDim.x > 32;
+    if (ordered)
+    {
+        for (int base = 0; tid < 32 && base < nh; base += 32)
+        {
+            const int i = base + tid;
+            int *const at = single ? s_wv + i : w.s_wave + cb + i;
+            const int wv = i < nh ? *at : 0;
+            const unsigned same = __match_any_sync(0xffffffffu, wv);
+            int first = 0;
+            if (i < nh && tid == __ffs(same) - 1)
+            {
+                int *const cursor = wide ? w.s_wcnt + cb + wv - 1 : s_cnt + wv - 1;
+                first = *cursor;
+                *cursor = first + __popc(same);
+            }
+            first = __shfl_sync(0xffffffffu, first, __ffs(same) - 1);
+            if (i < nh)
+                *at = first + __popc(same & ((1u << tid) - 1u));
+            __syncwarp(); // the cursors are the next hits'
+        }
+        __syncthreads();
+    }
     for (int i = tid; i < nh; i += blockDim.x)
     {
         int c, a, b, wv;
@@ -549,7 +577,7 @@ __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, 
         }
         const ContactGeo g = load_geometry(w, c, a, b);
         const int pidx = w.cand_pidx[c];
-        const int pos = cb + (wide ? atomicAdd(w.s_wcnt + cb + wv - 1, 1) : atomicAdd(s_cnt + wv - 1, 1));
+        const int pos = cb + (ordered ? wv : (wide ? atomicAdd(w.s_wcnt + cb + wv - 1, 1) : atomicAdd(s_cnt + wv - 1, 1)));
         float4 k[9];
         contact_constants(g, dt, k);
 #pragma unroll
