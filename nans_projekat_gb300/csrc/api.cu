@@ -96,6 +96,7 @@ struct nans_world
 
     int narrow_bpsm = 0;     // GJK blocks per SM (0 = occupancy limit)
     bool long_gjk = false;   // the long GJK runs take a thread each, not a warp
+    bool sphere_gjk = false; // so many spheres that their GJK runs go on in the first pass
     bool pair_only = false; // so few pairs that the narrowphase is the pair tier's launch alone
     int cull_tiles = 1;      // cull by tiles (1) or one lane per pair (0)
     int gjk_cap_blocks = 1;  // GJK blocks the world's pairs can keep busy
@@ -565,6 +566,10 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     // 0.410 ms a step at 122,000 bodies, 0.223 against 0.208 at 34,000. Hulls of many points always
     // take a warp (0.351 against 0.522 ms at 53,000 bodies).
     w->long_gjk = ndyn >= 80000 && !large_hulls;
+    // The first GJK pass's form for spheres (k_gjk) from a quarter of the bodies on, half where hulls of many
+    // points, which it leaves out, are among the others (301 to 4,096 mixed scenes of a quarter spheres
+    // and a third hulls: 0.3 to 0.8 % slower with it).
+    w->sphere_gjk = ts > 0 && 4 * ts >= (large_hulls ? 2 : 1) * (long long)ndyn;
     d.gjk_warp = (w->flags & NANS_WORLD_GJK_WARP) ? 1 : 0;
     d.sm_count = w->sm_count;
     d.giant_blocks = std::min(giant_grid(w->sm_count), upto(1, INT32_MAX) < 4096 ? 16 : INT32_MAX);
@@ -709,7 +714,7 @@ cudaError_t enqueue_narrow(nans_world *w, bool beside)
         return cudaGetLastError();
     }
     cudaError_t e = cudaSuccess;
-    launch_gjk(narrow_grid(w), st, w->dw);
+    launch_gjk(narrow_grid(w), st, w->dw, w->sphere_gjk);
     if (beside)
     {
         e = cudaEventRecord(w->ev_fork, st);

@@ -947,9 +947,35 @@ struct RegSupport
     }
 };
 
-// GJK of candidate c from call `it` with the simplex (s0..s3, n points), for up to `budget` calls. The
-// simplex of a hit and of a run still evolving goes to the candidate's slot; `hull` tells of a shape
-// of more than eight points.
+constexpr int kGjkShort = 8;
+// A sphere resting on a box takes 9 to 12 calls as often as not. Where kGjkTogether lanes of a warp hold
+// such a pair that is still evolving after kGjkShort calls, they go on to kGjkSphere calls in place
+// instead of taking a warp each on the pair tier. Hulls of many points and boxes do not: their runs are
+// longer. In worlds of many spheres (launch_gjk): 2,000 scenes of 20 spheres on the ground 291 -> 127 us a
+// step, 300 of them 114 -> 102, 100,000 scenes of a box and a sphere 787 -> 679, 50,000 of three boxes and
+// a sphere 661 -> 599. With one sphere among 32 boxes the lanes that wait cost more (1,000 such scenes
+// 169 -> 175), and the code alone 0.3 % of a step of 16,384 stacks, so those keep the plain form.
+constexpr int kGjkSphere = 12, kGjkTogether = 4;
+
+struct SphereCalls
+{
+    bool sphere; // a sphere and a shape of at most eight points
+    __device__ __forceinline__ bool operator()(int &budget) const
+    {
+        if (budget != kGjkShort)
+            return false;
+        const unsigned m = __ballot_sync(__activemask(), sphere);
+        if (!sphere || __popc(m) < kGjkTogether)
+            return false;
+        budget = kGjkSphere;
+        return true;
+    }
+};
+
+// GJK of candidate c from call `it` with the simplex (s0..s3, n points), for up to `budget` calls
+// (SPHERES: or as SphereCalls says). The simplex of a hit and of a run still evolving goes to the
+// candidate's slot; `hull` tells of a shape of more than eight points.
+template <bool SPHERES>
 __device__ __forceinline__ int gjk_run(const DevWorld &w, int c, int ia, int ib, int budget, GV &s0, GV &s1, GV &s2,
                                        GV &s3, int &n, int &it, bool &hull)
 {
@@ -961,7 +987,12 @@ __device__ __forceinline__ int gjk_run(const DevWorld &w, int c, int ia, int ib,
     if (rb)
         load_verts8(w.verts, B.off, VB);
     hull = max(A.npts, B.npts) > 8;
-    const int g = gjk_from_with(RegSupport{w.verts, A, B, ra, rb, VA, VB}, A, B, s0, s1, s2, s3, n, it, budget);
+    const RegSupport support{w.verts, A, B, ra, rb, VA, VB};
+    int g;
+    if constexpr (SPHERES)
+        g = gjk_from_with(support, A, B, s0, s1, s2, s3, n, it, budget, SphereCalls{!hull && min(A.npts, B.npts) == 0});
+    else
+        g = gjk_from_with(support, A, B, s0, s1, s2, s3, n, it, budget);
     if (g == G_FOUND || g == G_BUDGET)
         store_simplex(w, c, s0, s1, s2, s3);
     return g;
@@ -973,12 +1004,11 @@ __device__ __forceinline__ int gjk_run(const DevWorld &w, int c, int ia, int ib,
 // 99.5 -> 96 for 1,024 of 33 boxes); each lane runs GJK
 // (budget kGjkShort calls); GJKs that need more calls go to the long pass, so that the rare
 // long GJK runs share warps with each other instead of stalling 31 finished lanes.
-constexpr int kGjkShort = 8;
 constexpr int kGjkThreads = 128;
 // four blocks per SM (at most 128 registers, room for both shapes' vertices): measured best
 // against 5 and 6 (which spill the vertices) on the stack workload. Bound by issue (0.5 a cycle and
 // scheduler) and by the chain of loads before a batch (half of the stalls); 146 us a step of 16,384 stacks.
-__global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
+template <bool SPHERES> __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
 {
     const int lane = threadIdx.x & 31;
     const int n = *w.n_cand;
@@ -1018,7 +1048,7 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(DevWorld w)
             {
                 int np = 0, it = 0;
                 bool hull;
-                const int g = gjk_run(w, c, ia, ib, kGjkShort, s0, s1, s2, s3, np, it, hull);
+                const int g = gjk_run<SPHERES>(w, c, ia, ib, kGjkShort, s0, s1, s2, s3, np, it, hull);
                 if (g == G_NOHIT)
                     w.hit[c] = 0;
                 enqueue_pair(w, c, np | (it << 8), false, g == G_BUDGET);
@@ -1046,7 +1076,7 @@ __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk_long(DevWorld w)
         load_simplex(w, q.x, s0, s1, s2, s3);
         int np = q.y & 0xff, it = q.y >> 8;
         bool hull;
-        const bool hit = gjk_run(w, q.x, w.cand_a[q.x], w.cand_b[q.x], 65, s0, s1, s2, s3, np, it, hull) == G_FOUND;
+        const bool hit = gjk_run<false>(w, q.x, w.cand_a[q.x], w.cand_b[q.x], 65, s0, s1, s2, s3, np, it, hull) == G_FOUND;
         if (!hit)
             w.hit[q.x] = 0;
         w.long_cand[i] = make_int2(hit ? q.x : -1, kPairEpa);
@@ -1536,7 +1566,7 @@ int narrow_blocks_per_sm(int warps)
 {
     (void)warps;
     int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_gjk, kGjkThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_gjk<false>, kGjkThreads, 0);
     return per;
 }
 
@@ -1575,12 +1605,15 @@ int tier_priority()
     return prio;
 }
 
-void launch_gjk(int grid, cudaStream_t st, const DevWorld &w)
+// spheres: the form for worlds of many of them.
+void launch_gjk(int grid, cudaStream_t st, const DevWorld &w, bool spheres)
 {
     if (w.gjk_warp)
         k_gjk_warp<<<gjk_warp_grid(w), kGjkWarpThreads, 0, st>>>(w);
+    else if (spheres)
+        k_gjk<true><<<grid, kGjkThreads, 0, st>>>(w);
     else
-        k_gjk<<<grid, kGjkThreads, 0, st>>>(w);
+        k_gjk<false><<<grid, kGjkThreads, 0, st>>>(w);
 }
 
 void launch_gjk_long(int grid, cudaStream_t st, const DevWorld &w) { k_gjk_long<<<grid, kGjkThreads, 0, st>>>(w); }

@@ -146,16 +146,21 @@ __device__ __forceinline__ bool gjk_direction(VX &s0, VX &s1, VX &s2, VX &s3, in
 
 // CheckCollision's GJK loop (at most 65 EvolveSimplex calls) from call `it` with the simplex
 // (s0..s3, n points). With budget < 65 it stops before call `budget` and returns G_BUDGET if
-// the simplex is still evolving; (simplex, n, it) then resume it exactly.
-template <class Support>
+// the simplex is still evolving and more(budget) does not raise the budget; (simplex, n, it) then
+// resume it exactly.
+struct NoMoreCalls
+{
+    __device__ __forceinline__ bool operator()(int &) const { return false; }
+};
+template <class Support, class More = NoMoreCalls>
 __device__ __forceinline__ int gjk_from_with(const Support &support, const Shape &A, const Shape &B, GV &s0, GV &s1,
-                                             GV &s2, GV &s3, int &n, int &it, int budget)
+                                             GV &s2, GV &s3, int &n, int &it, int budget, const More &more = More())
 {
     const v3 dir0 = normalize3(B.p - A.p);
     int res = G_EVOLVING;
     for (; it <= 64; ++it)
     {
-        if (it >= budget)
+        if (it >= budget && !more(budget))
             return G_BUDGET;
         v3 dir = dir0;
         if (gjk_direction(s0, s1, s2, s3, n, dir))

@@ -118,7 +118,7 @@ enum PairPart
     PAIRS_BACK = 1,  // what the per-thread EPA left over
     PAIRS_ALL = 2,   // every candidate, in place of the GJK and per-thread EPA passes
 };
-void launch_gjk(int grid, cudaStream_t st, const DevWorld &w);
+void launch_gjk(int grid, cudaStream_t st, const DevWorld &w, bool spheres);
 void launch_gjk_long(int grid, cudaStream_t st, const DevWorld &w);
 void launch_epa_tiny(cudaStream_t st, const DevWorld &w);
 void launch_pair_warp(cudaStream_t st, const DevWorld &w, int part);
