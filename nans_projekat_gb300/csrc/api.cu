@@ -560,6 +560,12 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     // Steps of up to 16 candidates per SM give each pair a warp from the start of its GJK (136 against
     // 142 us a step at 2,000 candidates; 197 against 162 at 6,400: then a thread per pair).
     d.pair_max = 16 * w->sm_count;
+    // Above 400 candidates per SM the EPAs of hulls of many points (6 of 10 of a mixed scene's) keep the SMs
+    // busy with a thread each, below a warp's shorter chain wins. A warp and a thread each, us a step: hulls
+    // of 12 points 134 and 132 at 24,800 candidates, 186 and 159 at 49,600, 330 and 263 at 103,000, 657 and
+    // 502 at 248,000; of 8 to 32 points 237 and 249 at 49,000, 408 and 372 at 98,000, 685 and 595 at 197,000;
+    // of 30 points 187 and 209 at 22,000, 359 and 323 at 65,000; of 200 points 739 and 823 at 60,000.
+    d.hull_max = 400 * w->sm_count;
     w->pair_only = pair_acc <= d.pair_max && !(w->flags & NANS_WORLD_GJK_WARP);
     // The long GJK runs (~1.5 % of the candidates) take a thread each in worlds of many boxes and
     // spheres, where a warp each costs more issue slots than the shorter chain saves: 0.371 against

@@ -903,7 +903,8 @@ __device__ __forceinline__ void enqueue_pair(const DevWorld &w, int c, int state
 // took more than kEpaLongIters iterations at its last step fill the queue from the back (count in
 // work counter 9), the others from the front (work counter 10): the per-thread EPA pass takes
 // the long ones first, so that the lanes of a warp run EPAs of similar length. Pairs whose last
-// EPA would not have fitted the per-thread polytope go to the pair tier at once.
+// EPA would not have fitted the per-thread polytope go to the pair tier at once, and so do those with a
+// hull of more than eight points (`hull`) in steps of up to hull_max candidates.
 constexpr int kEpaLongIters = 4;
 constexpr int kEpaTinyIters = kTinyV - 3; // iterations a regular EPA can have on the per-thread polytope
 __device__ __forceinline__ void enqueue_epa(const DevWorld &w, int c, bool hit, bool hull)
@@ -1052,7 +1053,7 @@ template <bool SPHERES> __global__ void __launch_bounds__(kGjkThreads, 4) k_gjk(
                 if (g == G_NOHIT)
                     w.hit[c] = 0;
                 enqueue_pair(w, c, np | (it << 8), false, g == G_BUDGET);
-                enqueue_epa(w, c, g == G_FOUND, hull);
+                enqueue_epa(w, c, g == G_FOUND, hull && n <= w.hull_max);
             }
         }
         base = next;

@@ -105,6 +105,7 @@ struct DevWorld
     int tiny_blocks;                    // per-thread EPA grid (resident blocks on every SM)
     int pair_blocks;                   // pair-tier grid (resident blocks on every SM)
     int pair_max;                      // steps of up to this many candidates run on the pair tier alone
+    int hull_max;                      // and of up to this many, the EPAs of hulls of many points
     int gjk_warp;                       // 1: GJK with one warp per pair (NANS_WORLD_GJK_WARP)
     int sm_count;
     int ovf_cap;                        // block-EPA queue capacity
