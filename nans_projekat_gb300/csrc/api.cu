@@ -56,6 +56,10 @@ constexpr int kTuneSteps = 20;       // timed steps per autotuner candidate
 } // namespace
 
 constexpr size_t kHostStage = 64 * 1024; // bytes a world stages small downloads in
+constexpr int kHostWords = 4;            // words a world reads counts and status back into
+constexpr int kPageableReads = 2;        // small reads of a world before it takes page-locked memory
+constexpr int kCounterWords = 128;       // device words of a world's counters
+static_assert(kWorkCounters <= 32, "the work counters' place among the counters");
 
 struct nans_world
 {
@@ -82,9 +86,10 @@ struct nans_world
     float *d_rec_cube = nullptr, *d_rec_sphere = nullptr, *d_rec_floor = nullptr;
     float *d_pairs_out = nullptr;
     int pairs_out_cap = 0;
-    int *h_words = nullptr; // page-locked: status word, counts read back after a step; [2] a status to set
-    unsigned char *h_stage = nullptr; // page-locked, kHostStage bytes: small downloads in one wait
-    int *d_small = nullptr; // [0] pair count for k_pairs_out, [1] contact count
+    int words[kHostWords] = {};
+    int *h_words = words;   // status word, counts read back after a step; [2] a status to set (page_locked)
+    unsigned char *h_stage = nullptr; // page-locked, kHostStage bytes and h_words: small downloads in one wait
+    int small_reads = 0;
     float4 *d_snap = nullptr;
 
     bool uploaded = false;
@@ -497,23 +502,25 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
         (rc = dalloc(w, L, &d.pair_mask, (size_t)word_acc)) || (rc = dalloc(w, L, &p_wscene, (size_t)word_acc)) ||
         (rc = dalloc(w, L, &p_tiles, tiles.size())) || (rc = dalloc(w, L, &p_rest, rest_tasks.size())) ||
         (rc = dalloc(w, L, &d.epa_hist, (size_t)word_acc * 32)) ||
-        (rc = dalloc(w, L, &d.cull_state, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.cull_total, 1)) ||
-        (rc = dalloc(w, L, &d.n_cand, 3)) ||
+        (rc = dalloc(w, L, &d.cull_state, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.n_cand, kCounterWords)) ||
         (rc = dalloc(w, L, &d.cand_begin, S)) || (rc = dalloc(w, L, &d.cand_end, S)) ||
         (rc = dalloc(w, L, &d.scene_late, S)) || (rc = dalloc(w, L, &d.late_list, S)) ||
-        (rc = dalloc(w, L, &d.work_counter, kWorkCounters)) ||
         (rc = dalloc(w, L, &d.ovf_cand, kEpaOverflowCap)) || (rc = dalloc(w, L, &d.med_cand, kEpaMediumCap)) ||
         (rc = dalloc(w, L, &d.epa_arena, epa_big_bytes())) ||
         (rc = dalloc(w, L, &d.giant_scratch, epa_giant_scratch_bytes())) ||
         (rc = dalloc(w, L, &d.blk_arena, epa_block_bytes() * (size_t)(kBlockPerSm * w->sm_count))) ||
         (rc = dalloc(w, L, &d.giant_cand, kGiantQueueCap)) || (rc = dalloc(w, L, &d.handover, kHandoverSlots)) ||
-        (rc = dalloc(w, L, &d.epa_stats, 8)) || (rc = dalloc(w, L, &d.check, 4)) ||
         (rc = dalloc(w, L, &w->d_rec_cube, (size_t)61 * tc)) || (rc = dalloc(w, L, &w->d_rec_sphere, (size_t)37 * ts)) ||
-        (rc = dalloc(w, L, &w->d_rec_floor, (size_t)61 * S)) || (rc = dalloc(w, L, &w->d_small, 2)) ||
-        (rc = dalloc(w, L, &d.s_last, 1)))
+        (rc = dalloc(w, L, &w->d_rec_floor, (size_t)61 * S)))
         return rc;
-    d.status = reinterpret_cast<unsigned *>(d.n_cand + 1); // side by side: one copy reads them
+    // The counters in one allocation (each costs some 25 us of a world's life), those that the step's blocks
+    // count in on lines of their own; the first words side by side, so that one copy reads them.
+    d.status = reinterpret_cast<unsigned *>(d.n_cand + 1);
     d.cull_max = d.n_cand + 2;
+    d.cull_total = d.n_cand + 3;
+    d.work_counter = d.n_cand + 32;
+    d.epa_stats = reinterpret_cast<unsigned *>(d.n_cand + 64);
+    d.check = d.n_cand + 96;
     // no EPA seen yet: every pair starts in the short-EPA part of the queue
     CK(cudaMemset(d.epa_hist, 0, std::max(1LL, word_acc * 32)));
     // world vertices are written by the first step; zero until then (the renderer reads them)
@@ -622,12 +629,8 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     if (ts)
         CK(cudaMemcpyAsync(w->d_rec_sphere, spheres, ts * sizeof(nans_sphere), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(w->d_rec_floor, floors, S * sizeof(nans_cube), cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(d.status, 0, sizeof(unsigned), st));
     CK(cudaMemsetAsync(d.giant_scratch, 0, epa_giant_scratch_bytes(), st));
-    CK(cudaMemsetAsync(d.epa_stats, 0, 8 * sizeof(unsigned), st));
-    CK(cudaMemsetAsync(d.check, 0, 4 * sizeof(int), st));
-    CK(cudaMemsetAsync(d.n_cand, 0, sizeof(int), st));
-    CK(cudaMemsetAsync(d.cull_max, 0, sizeof(int), st));
+    CK(cudaMemsetAsync(d.n_cand, 0, kCounterWords * sizeof(int), st));
     CK(cudaMemsetAsync(d.cand_begin, 0, S * sizeof(int), st));
     CK(cudaMemsetAsync(d.cand_end, 0, S * sizeof(int), st));
     CK(cudaMemsetAsync(d.scene_late, 0, S * sizeof(int), st));
@@ -880,7 +883,25 @@ cudaError_t enqueue_fused_conditional(nans_world *w, float pending_dt, float dt,
     return et != cudaSuccess ? et : e;
 }
 
-// Sets the status word on the world's stream; a page-locked word of the world carries it.
+// Whether small reads go through the world's page-locked memory, which it takes at its third: a read from
+// there saves 10 to 35 us, but the memory costs 250 us to take and give back where the process holds none
+// (a world's life of one step and one download took 2.2 ms with it and 1.97 without). Counts one read.
+bool page_locked(nans_world *w)
+{
+    if (!w->h_stage && w->small_reads <= kPageableReads && ++w->small_reads > kPageableReads)
+    {
+        if (cudaMallocHost(&w->h_stage, kHostStage + kHostWords * sizeof(int)) == cudaSuccess)
+            w->h_words = reinterpret_cast<int *>(w->h_stage + kHostStage);
+        else
+        {
+            cudaGetLastError(); // the world goes on without
+            w->h_stage = nullptr;
+        }
+    }
+    return w->h_stage != nullptr;
+}
+
+// Sets the status word on the world's stream; a word of the world carries it.
 int set_status(nans_world *w, unsigned status)
 {
     w->h_words[2] = (int)status;
@@ -905,6 +926,7 @@ int step_eager(nans_world *w, float dt, bool check_capacity)
     CK(cudaGetLastError());
     if (check_capacity)
     {
+        page_locked(w);
         CK(cudaMemcpyAsync(w->h_words, d.status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         const unsigned status = (unsigned)w->h_words[0];
@@ -937,6 +959,7 @@ int status_code(nans_world *w, unsigned status);
 
 int check_status(nans_world *w)
 {
+    page_locked(w);
     CK(cudaMemcpyAsync(w->h_words, w->dw.status, sizeof(unsigned), cudaMemcpyDeviceToHost, w->stream));
     CK(cudaStreamSynchronize(w->stream));
     return status_code(w, (unsigned)w->h_words[0]);
@@ -1248,6 +1271,7 @@ int plain_steps(nans_world *w, float dt, uint32_t nsteps)
         for (uint32_t i = 0; i < nsteps; ++i)
             if ((rc = plain_step(w, dt)))
                 return rc;
+        page_locked(w);
         CK(cudaMemcpyAsync(w->h_words, d.status, 2 * sizeof(int), cudaMemcpyDeviceToHost, st)); // and cull_max
         CK(cudaStreamSynchronize(st));
         const unsigned hdr[2] = {(unsigned)w->h_words[0], (unsigned)w->h_words[1]};
@@ -1351,6 +1375,7 @@ int diff_step(nans_world *w, float dt, bool graph)
         if ((rc = ensure_graph_tape(w, dt)))
             return rc;
         CK(cudaGraphLaunch(w->gexec_t, st));
+        page_locked(w);
         CK(cudaMemcpyAsync(w->h_words, d.n_cand, 2 * sizeof(int), cudaMemcpyDeviceToHost, st)); // and the status
         CK(cudaStreamSynchronize(st));
         if (may_grow && (w->h_words[1] & (int)ST_CANDIDATES))
@@ -1377,6 +1402,7 @@ int diff_step(nans_world *w, float dt, bool graph)
         }
         if ((rc = step_eager(w, dt, true)))
             return rc;
+        page_locked(w);
         CK(cudaMemcpyAsync(w->h_words, d.n_cand, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
     }
@@ -1430,10 +1456,6 @@ int nans_world_create(const nans_world_desc *desc, nans_world **out)
     if (e == cudaSuccess)
         e = cudaEventCreateWithFlags(&w->ev_pairs, cudaEventDisableTiming);
     if (e == cudaSuccess)
-        e = cudaMallocHost(&w->h_words, 4 * sizeof(int));
-    if (e == cudaSuccess)
-        e = cudaMallocHost(&w->h_stage, kHostStage);
-    if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&w->sm_count, cudaDevAttrMultiProcessorCount, w->device);
     if (e == cudaSuccess)
         e = (cudaError_t)narrow_kernel_attrs();
@@ -1451,10 +1473,6 @@ int nans_world_create(const nans_world_desc *desc, nans_world **out)
             cudaEventDestroy(w->ev_join);
         if (w->ev_pairs)
             cudaEventDestroy(w->ev_pairs);
-        if (w->h_words)
-            cudaFreeHost(w->h_words);
-        if (w->h_stage)
-            cudaFreeHost(w->h_stage);
         delete w;
         return fail(NANS_ERR_CUDA, std::string("create: ") + cudaGetErrorString(e));
     }
@@ -1482,8 +1500,6 @@ int nans_world_destroy(nans_world *w)
         cudaFree(p);
     if (w->d_tape)
         cudaFree(w->d_tape);
-    if (w->h_words)
-        cudaFreeHost(w->h_words);
     if (w->h_stage)
         cudaFreeHost(w->h_stage);
     if (w->stream)
@@ -1738,7 +1754,7 @@ int nans_world_download(nans_world *w, nans_cube *cubes, nans_sphere *spheres, n
     const float *src[3] = {w->d_rec_cube, w->d_rec_sphere, w->d_rec_floor};
     const size_t bytes[3] = {w->n_cubes * sizeof(nans_cube), w->n_spheres * sizeof(nans_sphere),
                              w->n_scenes * sizeof(nans_cube)};
-    const bool staged = bytes[0] + bytes[1] + bytes[2] <= kHostStage;
+    const bool staged = bytes[0] + bytes[1] + bytes[2] <= kHostStage && page_locked(w);
     float *pack[3] = {w->d_rec_cube, w->d_rec_sphere, nullptr};
     size_t at = 0;
     for (int i = 0; staged && i < 3; ++i)
@@ -2031,7 +2047,7 @@ int nans_world_get_state_arrays(nans_world *w, float *position, float *angles, f
         if (dst[q])
             mask |= 1 << q;
     // a small world's arrays are written to page-locked memory by the kernel, without a copy
-    const bool staged = 4 * n3 * sizeof(float) <= kHostStage;
+    const bool staged = 4 * n3 * sizeof(float) <= kHostStage && page_locked(w);
     if ((mask || w->pending) && n3)
         k_state_out<<<nb, kSweepThreads, 0, st>>>(w->dw, w->pending_dt, w->pending,
                                                   staged ? (float *)w->h_stage : w->d_state_stage, w->d_body_rec,
@@ -2071,9 +2087,13 @@ int nans_get_pairs(nans_world *w, uint32_t scene, nans_contact_pair *out, uint32
         w->pairs_out_cap = (int)std::max<uint32_t>(cap, 1);
     }
     // the count, and a list that fits the page-locked buffer, are written there without a copy
-    const bool staged = out && cap && cap * sizeof(nans_contact_pair) <= kHostStage;
-    k_pairs_out<<<1, 256, 0, st>>>(w->dw, (int)scene, staged ? (float *)w->h_stage : w->d_pairs_out, (int)cap, w->h_words);
+    const bool locked = page_locked(w);
+    const bool staged = locked && out && cap && cap * sizeof(nans_contact_pair) <= kHostStage;
+    int *const count_out = locked ? w->h_words : w->dw.n_cand + 4;
+    k_pairs_out<<<1, 256, 0, st>>>(w->dw, (int)scene, staged ? (float *)w->h_stage : w->d_pairs_out, (int)cap, count_out);
     CK(cudaGetLastError());
+    if (!locked)
+        CK(cudaMemcpyAsync(w->h_words, count_out, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     const int n = w->h_words[0];
     *count = (uint32_t)n;

@@ -137,7 +137,6 @@ struct DevWorld
                                         // the narrowphase, per candidate: the GJK simplex of a hit.
                                         // Field by field (slot_k): the slots of neighbouring
                                         // threads lie side by side
-    int *s_last;                        // per body: last wave touching it
     int solve_rounds;                   // 1: the solver labels in rounds (two words a body fit its memory)
     int solve_cache;                    // scenes of up to this many bodies solve their waves on
                                         // a shared-memory copy of their velocities
