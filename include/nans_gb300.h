@@ -137,7 +137,7 @@ typedef struct nans_contact_pair
                                       tiers and the late solve pass. Same results. For worlds of a
                                       few small scenes, where the staged step's launch chain is
                                       the cost (the reference's own scene); a world with a scene of
-                                      more than 12 bodies or more scenes than the GPU has SMs takes
+                                      more than 14 bodies or more than two scenes per SM takes
                                       the staged kernels, which are faster there. Scenes of at most 1,024
                                       bodies; the candidate buffers hold every pair (the
                                       max_candidates request is raised to that); not with

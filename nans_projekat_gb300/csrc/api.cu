@@ -559,11 +559,12 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     d.tiny_blocks = upto(64, epa_tiny_grid(w->sm_count));
     d.pair_blocks = upto(2, pair_warp_grid(w->sm_count));
     // The fused step runs a scene on one block, so it pays while a scene's pairs go through the block's
-    // warps in a few turns and every scene has an SM. Fused and staged, us a step of a call of 40 steps:
-    // one scene of 4 bodies 43 and 50, of 9 58 and 57, of 16 58 and 53, of 24 60 and 54; 30 scenes of 4
-    // 73 and 78, of 12 78 and 74, of 24 97 and 84; 150 scenes of 4 75 and 84, of 12 88 and 94, of 24 108
-    // and 106. One step a call: 52 and 63 at 4 bodies, 65 and 66 at 9, 70 and 64 at 24.
-    w->fused_small = w->fused && max_bodies <= kSceneStepBodies && S <= w->sm_count;
+    // warps in a few turns and the scenes run side by side. Fused and staged, us a step of a call of 40
+    // steps: one scene of 4 bodies 31 and 44, of 14 41 and 50, of 16 48 and 52; 24 scenes of 9 73 and
+    // 77, of 14 69 and 76; 300 of 9 93 and 125, of 14 81 and 105; 400 of 14 104 and 110. It took 0.69 to
+    // 0.99 of the staged time for 4 to 14 bodies and 1 to 300 scenes, a step or 40 a call and in graphs of
+    // 40; with 16 bodies up to 1.04 (4 to 16 scenes), and with 800 scenes and more the blocks queue.
+    w->fused_small = w->fused && max_bodies <= kSceneStepBodies && S <= 2 * w->sm_count;
     // Steps of up to 16 candidates per SM give each pair a warp from the start of its GJK (136 against
     // 142 us a step at 2,000 candidates; 197 against 162 at 6,400: then a thread per pair).
     d.pair_max = 16 * w->sm_count;

@@ -1364,13 +1364,14 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32) k_epa_medium(
 
 
 // ---------------------------------------------------------------------------------------
-// The fused per-scene step (NANS_WORLD_FUSED_STEP): after the sweep, one launch in which a
-// block of kSceneThreads threads takes a scene at a time (largest first) and runs its whole
+// The fused per-scene step (NANS_WORLD_FUSED_STEP, scenes of up to kSceneStepBodies bodies): after the
+// sweep, one launch in which a block of kSceneThreads threads runs a scene's whole
 // detect-and-solve sequence, each phase on the block:
-//   (1) the cull: the scene's pairs in the reference's order (code/nans.cpp:1355-1535), kept
-//       when their inflated boxes meet (k_cull_place's test), compacted in order by block scans
-//       into the scene's own slots of the pair space (from sc_word0 * 32: the candidate
-//       buffers of such a world hold every pair, so no scan across scenes is needed);
+//   (1) the cull: the scene's pairs, one a thread, in the reference's order
+//       (code/nans.cpp:1355-1535), kept when their inflated boxes meet (k_cull_place's test),
+//       compacted in order by a block scan into the scene's own slots of the pair space (from
+//       sc_word0 * 32: the candidate buffers of such a world hold every pair, so no scan across
+//       scenes is needed);
 //   (2) GJK and EPA, a warp per candidate (pair_warp);
 //   (3) the EPAs that outgrew its registers, one per warp on the warp tier's polytope (epa_run);
 //   (4) the solve (solve_scene), unless an EPA outgrew the warp tier: that pair goes to the
@@ -1384,11 +1385,12 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32) k_epa_medium(
 constexpr int kSceneThreads = 256;
 constexpr int kSceneWarpEpas = 2; // warps of the block that run warp-tier EPAs (shared memory)
 static_assert(kSceneThreads % 32 == 0 && kSceneThreads <= kWaveChunk, "scene step block size");
+static_assert(kSceneStepBodies * (kSceneStepBodies + 1) / 2 <= kSceneThreads, "a thread per pair");
 // the block's dynamic shared memory stays within the 48 KB a launch gets without an opt-in
 static_assert((kSceneThreads / 32) * sizeof(WarpEpa) <= 48 * 1024 &&
                   kSceneWarpEpas * sizeof(EpaFast) <= 48 * 1024 &&
-                  (size_t)(kSceneStepMaxBodies + 1) * 2 * sizeof(float4) <= 48 * 1024 &&
-                  4 * kWaveChunk * sizeof(int) + 2 * kSceneStepMaxBodies * sizeof(int) <= 48 * 1024,
+                  (size_t)(kSceneStepBodies + 1) * 2 * sizeof(float4) <= 48 * 1024 &&
+                  4 * kWaveChunk * sizeof(int) + 2 * kSceneStepBodies * sizeof(int) <= 48 * 1024,
               "scene step shared memory");
 
 size_t scene_step_smem(size_t solve_bytes)
@@ -1405,133 +1407,100 @@ __global__ void __launch_bounds__(kSceneThreads) k_scene_step(DevWorld w, float 
     EpaFast *const epa = reinterpret_cast<EpaFast *>(smem_raw);
     float4 *const s_dyn = reinterpret_cast<float4 *>(smem_raw);
     __shared__ int sh[32];
-    __shared__ int s_q, s_nw, s_late, s_maxw;
+    __shared__ int s_nw, s_late, s_maxw;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (;;)
+    if (tid == 0)
     {
-        if (tid == 0)
-        {
-            s_q = atomicAdd(w.work_counter + 14, 1);
-            s_nw = 0;
-            s_late = 0;
-        }
-        __syncthreads();
-        const int q = s_q;
-        if (q >= w.n_scenes)
-            break;
-        const int s = w.sc_order[q];
-        const int c0 = w.sc_cube0[s], nc = w.sc_nc[s], ns = w.sc_ns[s];
-        const long long np = scene_pair_count(nc, ns);
-        const int cb = w.sc_word0[s] * 32;
-        // (1) the cull, eight consecutive pairs a thread between the block scans
-        int nk = 0;
-        for (long long base = 0; base < np; base += 8 * kSceneThreads)
-        {
-            const long long k0 = base + 8ll * tid;
-            int t0 = 0, i0 = 0, j0 = 0;
-            unsigned m = 0u;
-            if (k0 < np)
-            {
-                decode_pair(k0, nc, ns, t0, i0, j0);
-                const int cnt = (int)min(8ll, np - k0);
-                for (int o = 0; o < cnt; ++o)
-                {
-                    int type, i, j, a, b;
-                    pair_after(k0, nc, ns, t0, i0, j0, o, type, i, j);
-                    pair_ids(w, s, c0, nc, type, i, j, a, b);
-                    bool keep = true;
-                    if (!all_pairs)
-                    {
-                        const float4 la = __ldg(w.box_lo + a), ha = __ldg(w.box_hi + a);
-                        const float4 lb = __ldg(w.box_lo + b), hb = __ldg(w.box_hi + b);
-                        keep = la.x <= hb.x && lb.x <= ha.x && la.y <= hb.y && lb.y <= ha.y && la.z <= hb.z &&
-                               lb.z <= ha.z;
-                    }
-                    if (keep)
-                        m |= 1u << o;
-                }
-            }
-            int tot;
-            int pos = cb + nk + block_scan_excl(__popc(m), sh, &tot);
-            while (m)
-            {
-                const int o = __ffs(m) - 1;
-                m &= m - 1u;
-                int type, i, j, a, b;
-                pair_after(k0, nc, ns, t0, i0, j0, o, type, i, j);
-                pair_ids(w, s, c0, nc, type, i, j, a, b);
-                if (dev_check(w, pos < w.cand_cap, 20, pos, w.cand_cap))
-                {
-                    w.cand_a[pos] = a;
-                    w.cand_b[pos] = b;
-                    w.cand_meta[pos] = (s << 3) | type;
-                    w.cand_pidx[pos] = cb + (int)(k0 + o);
-                }
-                ++pos;
-            }
-            nk += tot;
-        }
-        const int ce = min(cb + nk, w.cand_cap);
-        if (tid == 0)
-        {
-            w.cand_begin[s] = cb;
-            w.cand_end[s] = ce;
-            w.scene_late[s] = 0;
-        }
-        __syncthreads(); // the last chunk's candidates, written after its scan
-        // (2) GJK and EPA, a warp per candidate; the EPAs that outgrow its registers go to
-        // s_wave[cb ..)
-        for (int c = cb + wid; c < ce; c += kSceneThreads / 32)
-        {
-            const int r = pair_warp(w, reinterpret_cast<WarpEpa *>(smem_raw)[wid], c, true, 0, 0, lane);
-            if (r == EPA_OVERFLOW && lane == 0)
-            {
-                w.hit[c] = 0;
-                atomicAdd(w.epa_stats + 6, 1u);
-                w.s_wave[cb + atomicAdd(&s_nw, 1)] = c;
-            }
-            __syncwarp();
-        }
-        __syncthreads(); // the pairs' polytopes' memory becomes the warp tier's
-        // (3) warp tier, from the simplex the GJK stored
-        const int nw = s_nw;
-        for (int i = wid; i < nw && wid < kSceneWarpEpas; i += kSceneWarpEpas)
-        {
-            EpaFast &E = epa[wid];
-            int cc = w.s_wave[cb + i];
-            if (!dev_check(w, cc >= cb && cc < ce, 22, cc, ce))
-                cc = -1;
-            if (cc < 0)
-                continue;
-            const Shape A = load_shape(w, w.cand_a[cc]), B = load_shape(w, w.cand_b[cc]);
-            GV g[4];
-            load_simplex(w, cc, g[0], g[1], g[2], g[3]);
-            v3 pa, pb, nn;
-            int4 ovf;
-            const int r = epa_run(w, E, A, B, g[0], g[1], g[2], g[3], pa, pb, nn, lane, ovf);
-            __syncwarp();
-            int qo = -1;
-            if (lane == 0)
-            {
-                if (r == EPA_OVERFLOW)
-                {
-                    qo = escalate(w, cc, true);
-                    s_late = 1;
-                }
-                else
-                    write_result(w, cc, r, pa, pb, nn);
-            }
-            qo = __shfl_sync(0xffffffffu, qo, 0);
-            if (qo >= 0 && qo < kHandoverSlots)
-                handover_put(w, E, qo, ovf, lane);
-            __syncwarp();
-        }
-        __syncthreads(); // the warps' polytopes' memory becomes the solver's
-        // (4) the solve, unless a pair of the scene went to the large tiers (the late pass)
-        if (!s_late)
-            solve_scene<false>(w, s, dt, s_dyn, sh, s_maxw);
-        __syncthreads();
+        s_nw = 0;
+        s_late = 0;
     }
+    const int s = w.sc_order[blockIdx.x];
+    const int c0 = w.sc_cube0[s], nc = w.sc_nc[s], ns = w.sc_ns[s];
+    const int cb = w.sc_word0[s] * 32;
+    // (1) the cull
+    int type = 0, a = 0, b = 0;
+    bool keep = false;
+    if (tid < (int)scene_pair_count(nc, ns))
+    {
+        int i, j;
+        decode_pair(tid, nc, ns, type, i, j);
+        pair_ids(w, s, c0, nc, type, i, j, a, b);
+        keep = true;
+        if (!all_pairs)
+        {
+            const float4 la = __ldg(w.box_lo + a), ha = __ldg(w.box_hi + a);
+            const float4 lb = __ldg(w.box_lo + b), hb = __ldg(w.box_hi + b);
+            keep = la.x <= hb.x && lb.x <= ha.x && la.y <= hb.y && lb.y <= ha.y && la.z <= hb.z && lb.z <= ha.z;
+        }
+    }
+    int nk;
+    const int pos = cb + block_scan_excl(keep ? 1 : 0, sh, &nk);
+    if (keep && dev_check(w, pos < w.cand_cap, 20, pos, w.cand_cap))
+    {
+        w.cand_a[pos] = a;
+        w.cand_b[pos] = b;
+        w.cand_meta[pos] = (s << 3) | type;
+        w.cand_pidx[pos] = cb + tid;
+    }
+    const int ce = min(cb + nk, w.cand_cap);
+    if (tid == 0)
+    {
+        w.cand_begin[s] = cb;
+        w.cand_end[s] = ce;
+        w.scene_late[s] = 0;
+    }
+    __syncthreads(); // the candidates
+    // (2) GJK and EPA, a warp per candidate; the EPAs that outgrow its registers go to
+    // s_wave[cb ..)
+    for (int c = cb + wid; c < ce; c += kSceneThreads / 32)
+    {
+        const int r = pair_warp(w, reinterpret_cast<WarpEpa *>(smem_raw)[wid], c, true, 0, 0, lane);
+        if (r == EPA_OVERFLOW && lane == 0)
+        {
+            w.hit[c] = 0;
+            atomicAdd(w.epa_stats + 6, 1u);
+            w.s_wave[cb + atomicAdd(&s_nw, 1)] = c;
+        }
+        __syncwarp();
+    }
+    __syncthreads(); // the pairs' polytopes' memory becomes the warp tier's
+    // (3) warp tier, from the simplex the GJK stored
+    const int nw = s_nw;
+    for (int i = wid; i < nw && wid < kSceneWarpEpas; i += kSceneWarpEpas)
+    {
+        EpaFast &E = epa[wid];
+        int cc = w.s_wave[cb + i];
+        if (!dev_check(w, cc >= cb && cc < ce, 22, cc, ce))
+            cc = -1;
+        if (cc < 0)
+            continue;
+        const Shape A = load_shape(w, w.cand_a[cc]), B = load_shape(w, w.cand_b[cc]);
+        GV g[4];
+        load_simplex(w, cc, g[0], g[1], g[2], g[3]);
+        v3 pa, pb, nn;
+        int4 ovf;
+        const int r = epa_run(w, E, A, B, g[0], g[1], g[2], g[3], pa, pb, nn, lane, ovf);
+        __syncwarp();
+        int qo = -1;
+        if (lane == 0)
+        {
+            if (r == EPA_OVERFLOW)
+            {
+                qo = escalate(w, cc, true);
+                s_late = 1;
+            }
+            else
+                write_result(w, cc, r, pa, pb, nn);
+        }
+        qo = __shfl_sync(0xffffffffu, qo, 0);
+        if (qo >= 0 && qo < kHandoverSlots)
+            handover_put(w, E, qo, ovf, lane);
+        __syncwarp();
+    }
+    __syncthreads(); // the warps' polytopes' memory becomes the solver's
+    // (4) the solve, unless a pair of the scene went to the large tiers (the late pass)
+    if (!s_late)
+        solve_scene<false>(w, s, dt, s_dyn, sh, s_maxw);
     // In a graph, the last block to finish opens the conditional node of the large tiers and the
     // late pass when a scene went late (work counter 13, counted by escalate); one call per launch.
     if (signal && tid == 0)
@@ -1542,15 +1511,11 @@ __global__ void __launch_bounds__(kSceneThreads) k_scene_step(DevWorld w, float 
     }
 }
 
-// The fused step's launch: resident blocks on every SM, no more than the world's scenes.
+// The fused step's launch: a block per scene.
 void launch_scene_step(const DevWorld &w, size_t solve_bytes, float dt, int all_pairs, cudaStream_t st,
                        cudaGraphConditionalHandle cond, int signal)
 {
-    const size_t smem = scene_step_smem(solve_bytes);
-    int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_scene_step, kSceneThreads, smem);
-    const int grid = std::max(1, std::min(w.n_scenes, std::max(1, per) * std::max(1, w.sm_count)));
-    k_scene_step<<<grid, kSceneThreads, smem, st>>>(w, dt, all_pairs, cond, signal);
+    k_scene_step<<<w.n_scenes, kSceneThreads, scene_step_smem(solve_bytes), st>>>(w, dt, all_pairs, cond, signal);
 }
 
 static size_t medium_smem(int warps) { return sizeof(EpaFast) * (size_t)warps; }

@@ -41,7 +41,7 @@ constexpr int kWaveChunk = 256;     // solver: candidates compacted and labelled
 constexpr size_t kSolveSmemMax = 200 * 1024; // solver: dynamic shared memory per block, at most
 constexpr int kMediumBlocksPerSm = 2;    // warp-tier EPA blocks per SM (shared memory allows three)
 constexpr int kSceneStepMaxBodies = 1024; // fused per-scene worlds: bodies per scene, at most
-constexpr int kSceneStepBodies = 12;     // fused per-scene step: larger scenes take the staged kernels
+constexpr int kSceneStepBodies = 14;     // fused per-scene step: larger scenes take the staged kernels
 
 // EPA capacities. Vertices: the GJK tetrahedron plus one support per EPA iteration (at most
 // 65, code/nans.cpp:804). Faces grow by two per iteration on a convex polytope, but the

@@ -145,7 +145,7 @@ class World:
     batch_step(dt, n, g)   the batched path: persistent kernels replayed from a CUDA graph
     fused_step=True        one detect-and-solve launch per step, a block per scene, in place of
                            the staged kernels where that is the faster, for a few scenes of up to
-                           12 bodies (same results; scenes of at most 1,024 bodies)
+                           14 bodies (same results; scenes of at most 1,024 bodies)
     """
 
     def __init__(self, device=0, all_pairs=False, max_candidates=0, strict_epa=False, giant_tier_only=False,
