@@ -30,7 +30,12 @@ sys.path.insert(0, ROOT)
 METRIC = "body-steps/s"
 UNIT = "body-steps/s"
 DT = np.float32(1.0 / 60.0)
-FUSED_MAX_BODIES = 1024           # NANS_WORLD_FUSED_STEP: bodies per scene, at most
+FUSED_MAX_BODIES = 14             # NANS_WORLD_FUSED_STEP: larger scenes take the staged kernels
+# the profiled stages: their kernels, and their keys in profiles/traffic.json
+STAGES = (("k_sweep", "k_sweep"), ("k_cull_tiles + k_cull_place", "cull"),
+          ("k_gjk + k_gjk_long + k_pair_warp + k_epa_tiny", "narrowphase"), ("k_epa_medium", "k_epa_medium"),
+          ("k_epa_block + k_epa_giant", "k_epa_large"), ("k_solve", "k_solve"))
+FUSED_LAUNCHES = (5, 5)           # launches_per_step() of a world that takes the fused kernel
 ALG_BYTES_SWEEP_BODY = 68 + 72     # read P,A,V,W,m,I,extents; write P,A,V,W,AABB
 ALG_BYTES_SWEEP_BOX_VERTS = 96     # world vertices written for the narrowphase
 # per body-step with the world vertices kept in registers: read P,A,V,W,F,T (72 B), m, I (8 B),
@@ -332,17 +337,19 @@ def single_scene_line(lib, device, scene, name, gpu_steps, cpu_steps):
         w.step(dt, gpu_steps)
         t_batch = (time.perf_counter() - t0) / gpu_steps
         graph_steps, eager_steps = w.path_counts()
+        taken = w.launches_per_step() == FUSED_LAUNCHES
         w.close()
-        return t_call, t_frame, t_batch, graph_steps, eager_steps
+        return t_call, t_frame, t_batch, graph_steps, eager_steps, taken
 
-    t_call, t_frame, t_batch, graph_steps, eager_steps = timed(False)
+    t_call, t_frame, t_batch, graph_steps, eager_steps, _ = timed(False)
     out = {"workload": name, "bodies": int(scene.n_bodies),
            "gpu_us_per_step": 1e6 * t_call, "gpu_us_per_step_with_download": 1e6 * t_frame,
            "gpu_us_per_step_one_call": 1e6 * t_batch,
            "gpu_path": "nans_step; %d of %d steps replayed from one-step CUDA graphs" % (
                graph_steps, graph_steps + eager_steps)}
     if scene.n_bodies <= FUSED_MAX_BODIES:
-        t_call, t_frame, t_batch, _, _ = timed(True)
+        t_call, t_frame, t_batch, _, _, taken = timed(True)
+        assert taken
         out["fused_step"] = {"gpu_us_per_step": 1e6 * t_call, "gpu_us_per_step_with_download": 1e6 * t_frame,
                              "gpu_us_per_step_one_call": 1e6 * t_batch,
                              "gpu_path": "nans_step on a NANS_WORLD_FUSED_STEP world (sweep + one detect-and-"
@@ -399,18 +406,23 @@ def fused_ab(lib, batch, device, warm=5, n=20):
     (NANS_WORLD_FUSED_STEP: after the sweep, one launch in which a block per scene culls, collides
     and solves) on identical windows: each world steps the same scenes from the upload (the
     results are the same bit for bit), then n steps from one CUDA graph are timed with CUDA
-    events. The whole workload and its scenes binned by size."""
+    events. The workload's first scenes of up to FUSED_MAX_BODIES bodies, as many as the name says:
+    worlds that take the fused kernel, which launches_per_step() tells."""
     import torch
-    bins = (("all", 0, 10 ** 9), ("4-16 bodies", 0, 16), ("17-64 bodies", 17, 64), ("65-256 bodies", 65, 10 ** 9))
+    small = [sc for sc in batch if sc.n_bodies <= FUSED_MAX_BODIES]
     out = {}
-    for name, lo, hi in bins:
-        sub = [sc for sc in batch if lo <= sc.n_bodies <= hi]
-        if not sub:
+    for count in (1, 24, 150, 300):
+        sub = small[:count]
+        if len(sub) < count:
             continue
         row = {"scenes": len(sub), "bodies": int(sum(sc.n_bodies for sc in sub))}
         for key, fused in (("staged_ms_per_step", False), ("fused_ms_per_step", True)):
             w = lib.World(device=device, fused_step=fused)
             w.upload_batch(sub)
+            if (w.launches_per_step() == FUSED_LAUNCHES) != fused:
+                row = None
+                w.close()
+                break
             w.batch_step(DT, warm, 1)
             w.prepare(DT, n)
             torch.cuda.synchronize()
@@ -423,8 +435,9 @@ def fused_ab(lib, batch, device, warm=5, n=20):
             row[key] = e0.elapsed_time(e1) / n
             assert w.path_counts()[0] >= n
             w.close()
-        row["fused_over_staged"] = row["fused_ms_per_step"] / row["staged_ms_per_step"]
-        out[name] = row
+        if row:
+            row["fused_over_staged"] = row["fused_ms_per_step"] / row["staged_ms_per_step"]
+            out["%d scenes of 4-%d bodies" % (count, FUSED_MAX_BODIES)] = row
     out["window"] = "steps %d-%d after the upload, one %d-step CUDA graph each" % (warm + 1, warm + n, n)
     return out
 
@@ -461,19 +474,25 @@ def secondary_measurements(lib, batch, device):
                          "sample": "every 256th scene of the workload, one world per scene, nans_step"}
     for wd in worlds:
         wd.close()
-    worlds = []
+    # the same with the fused step, on those of the scenes that take it
+    worlds, fused_bodies = [], 0
     for sc in sample:
         wd = lib.World(device=device, fused_step=True)
         wd.upload(sc)
+        if wd.launches_per_step() != FUSED_LAUNCHES:
+            wd.close()
+            continue
         wd.step(DT, 2)
         worlds.append(wd)
-    torch.cuda.synchronize()
-    t0 = time.perf_counter()
-    for wd in worlds:
-        wd.step(DT, n)
-    torch.cuda.synchronize()
-    t = time.perf_counter() - t0
-    out["plain_path"]["fused_step_value"] = bodies * n / t
+        fused_bodies += sc.n_bodies
+    if worlds:
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        for wd in worlds:
+            wd.step(DT, n)
+        torch.cuda.synchronize()
+        t = time.perf_counter() - t0
+        out["plain_path"]["fused_step"] = {"value": fused_bodies * n / t, "scenes": len(worlds), "bodies": fused_bodies}
     for wd in worlds:
         wd.close()
     # one large scene: 4,096 boxes + 512 spheres in a 64^3 m box, plain path
@@ -749,7 +768,7 @@ def run_ours(args):
     ends = w.timeline(DT, prof_steps)
     end_names = ["sweep", "cull", "gjk_and_thread_epa", "warp_epa (stream 2)", "large_epa (stream 2)",
                  "solve_pass0", "solve_pass1 (step end)"]
-    names = ["k_sweep", "k_cull (3 kernels)", "k_narrow_tiny", "k_epa_medium", "k_narrow_big (block + giant tiers)", "k_solve"]
+    names, traffic_keys = [n for n, _ in STAGES], [k for _, k in STAGES]
     dom = int(np.argmax(stage_ms))
     peak, peak_kind = measured_peaks()
     n_boxes = int(sum(len(s.cubes) for s in batch))
@@ -841,7 +860,7 @@ def run_ours(args):
                               "warp_tier_epas": epa["warp_tier"], "giant_tier_epas": epa["giant_tier"]},
             },
             "roofline": {"bound": "hbm", "kernel": names[dom], "achieved": achieved, "peak": peak,
-                         "unit": "GB/s", "frac": achieved / peak, "traffic": measured_traffic(names[dom]),
+                         "unit": "GB/s", "frac": achieved / peak, "traffic": measured_traffic(traffic_keys[dom]),
                          "peak_source": peak_kind + " hbm_gbs",
                          "bytes_per_launch": dom_bytes,
                          "stage_ms": {n: float(x) for n, x in zip(names, stage_ms)},
