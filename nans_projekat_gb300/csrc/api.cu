@@ -58,8 +58,6 @@ constexpr int kTuneSteps = 20;       // timed steps per autotuner candidate
 constexpr size_t kHostStage = 64 * 1024; // bytes a world stages small downloads in
 constexpr int kHostWords = 4;            // words a world reads counts and status back into
 constexpr int kPageableReads = 2;        // small reads of a world before it takes page-locked memory
-constexpr int kCounterWords = 128;       // device words of a world's counters
-static_assert(kWorkCounters <= 32, "the work counters' place among the counters");
 
 struct nans_world
 {
@@ -90,6 +88,7 @@ struct nans_world
     int *h_words = words;   // status word, counts read back after a step; [2] a status to set (page_locked)
     unsigned char *h_stage = nullptr; // page-locked, kHostStage bytes and h_words: small downloads in one wait
     int small_reads = 0;
+    int *d_pair_count = nullptr; // a contact list's length, before h_words is page-locked
     float4 *d_snap = nullptr;
 
     bool uploaded = false;
@@ -502,25 +501,22 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
         (rc = dalloc(w, L, &d.pair_mask, (size_t)word_acc)) || (rc = dalloc(w, L, &p_wscene, (size_t)word_acc)) ||
         (rc = dalloc(w, L, &p_tiles, tiles.size())) || (rc = dalloc(w, L, &p_rest, rest_tasks.size())) ||
         (rc = dalloc(w, L, &d.epa_hist, (size_t)word_acc * 32)) ||
-        (rc = dalloc(w, L, &d.cull_state, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.n_cand, kCounterWords)) ||
+        (rc = dalloc(w, L, &d.cull_state, std::max(1, w->cull_blocks))) || (rc = dalloc(w, L, &d.cull_total, 1)) ||
+        (rc = dalloc(w, L, &d.n_cand, 3)) ||
         (rc = dalloc(w, L, &d.cand_begin, S)) || (rc = dalloc(w, L, &d.cand_end, S)) ||
         (rc = dalloc(w, L, &d.scene_late, S)) || (rc = dalloc(w, L, &d.late_list, S)) ||
+        (rc = dalloc(w, L, &d.work_counter, kWorkCounters)) ||
         (rc = dalloc(w, L, &d.ovf_cand, kEpaOverflowCap)) || (rc = dalloc(w, L, &d.med_cand, kEpaMediumCap)) ||
         (rc = dalloc(w, L, &d.epa_arena, epa_big_bytes())) ||
         (rc = dalloc(w, L, &d.giant_scratch, epa_giant_scratch_bytes())) ||
         (rc = dalloc(w, L, &d.blk_arena, epa_block_bytes() * (size_t)(kBlockPerSm * w->sm_count))) ||
         (rc = dalloc(w, L, &d.giant_cand, kGiantQueueCap)) || (rc = dalloc(w, L, &d.handover, kHandoverSlots)) ||
+        (rc = dalloc(w, L, &d.epa_stats, 8)) || (rc = dalloc(w, L, &d.check, 4)) ||
         (rc = dalloc(w, L, &w->d_rec_cube, (size_t)61 * tc)) || (rc = dalloc(w, L, &w->d_rec_sphere, (size_t)37 * ts)) ||
-        (rc = dalloc(w, L, &w->d_rec_floor, (size_t)61 * S)))
+        (rc = dalloc(w, L, &w->d_rec_floor, (size_t)61 * S)) || (rc = dalloc(w, L, &w->d_pair_count, 1)))
         return rc;
-    // The counters in one allocation (each costs some 25 us of a world's life), those that the step's blocks
-    // count in on lines of their own; the first words side by side, so that one copy reads them.
-    d.status = reinterpret_cast<unsigned *>(d.n_cand + 1);
+    d.status = reinterpret_cast<unsigned *>(d.n_cand + 1); // side by side: one copy reads them
     d.cull_max = d.n_cand + 2;
-    d.cull_total = d.n_cand + 3;
-    d.work_counter = d.n_cand + 32;
-    d.epa_stats = reinterpret_cast<unsigned *>(d.n_cand + 64);
-    d.check = d.n_cand + 96;
     // no EPA seen yet: every pair starts in the short-EPA part of the queue
     CK(cudaMemset(d.epa_hist, 0, std::max(1LL, word_acc * 32)));
     // world vertices are written by the first step; zero until then (the renderer reads them)
@@ -630,8 +626,12 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     if (ts)
         CK(cudaMemcpyAsync(w->d_rec_sphere, spheres, ts * sizeof(nans_sphere), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(w->d_rec_floor, floors, S * sizeof(nans_cube), cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(d.status, 0, sizeof(unsigned), st));
     CK(cudaMemsetAsync(d.giant_scratch, 0, epa_giant_scratch_bytes(), st));
-    CK(cudaMemsetAsync(d.n_cand, 0, kCounterWords * sizeof(int), st));
+    CK(cudaMemsetAsync(d.epa_stats, 0, 8 * sizeof(unsigned), st));
+    CK(cudaMemsetAsync(d.check, 0, 4 * sizeof(int), st));
+    CK(cudaMemsetAsync(d.n_cand, 0, sizeof(int), st));
+    CK(cudaMemsetAsync(d.cull_max, 0, sizeof(int), st));
     CK(cudaMemsetAsync(d.cand_begin, 0, S * sizeof(int), st));
     CK(cudaMemsetAsync(d.cand_end, 0, S * sizeof(int), st));
     CK(cudaMemsetAsync(d.scene_late, 0, S * sizeof(int), st));
@@ -2090,7 +2090,7 @@ int nans_get_pairs(nans_world *w, uint32_t scene, nans_contact_pair *out, uint32
     // the count, and a list that fits the page-locked buffer, are written there without a copy
     const bool locked = page_locked(w);
     const bool staged = locked && out && cap && cap * sizeof(nans_contact_pair) <= kHostStage;
-    int *const count_out = locked ? w->h_words : w->dw.n_cand + 4;
+    int *const count_out = locked ? w->h_words : w->d_pair_count;
     k_pairs_out<<<1, 256, 0, st>>>(w->dw, (int)scene, staged ? (float *)w->h_stage : w->d_pairs_out, (int)cap, count_out);
     CK(cudaGetLastError());
     if (!locked)
