@@ -299,7 +299,7 @@ int nans_world_set_tuning(nans_world *world, const int32_t *in);
 
 /* Steps run since the last upload by nans_step and nans_batch_step, split into those replayed
  * from a CUDA graph and those launched kernel by kernel (the first step after an upload or a
- * set_state, and steps left over from whole graphs). No reference counterpart. */
+ * set_state, on the plain path unless the last such step was alike). No reference counterpart. */
 int nans_world_path_counts(nans_world *world, uint64_t *graph_steps, uint64_t *eager_steps);
 
 /* The project sine/cosine used by the Model rebuild, evaluated on the device (n values); it
@@ -328,7 +328,8 @@ int nans_device_sincos(const float *x, float *s, float *c, uint32_t n);
  * Per-body arrays are float[n][3] (d_mass: float[n]) in record order: the cubes of all scenes
  * in upload order, then the spheres. Per-scene arrays hold one float per scene. Input
  * pointers may be NULL (zero); output pointers may be NULL (not wanted). The tape stays valid
- * until the next step, upload, set_state or forward; the backward may run several times. */
+ * until the next step, upload, set_state or forward; the backward may run several times. The same
+ * rollout from the same state gives the same gradients, bit for bit. */
 typedef struct nans_diff_grads
 {
     const float *dl_position;  /* in: dL/d final Position */

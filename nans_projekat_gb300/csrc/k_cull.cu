@@ -8,7 +8,8 @@
 // skipping pairs whose inflated AABBs are disjoint:
 //   k_cull_tiles  the words' bits: cube-cube pairs by 32 x 32 tiles, the others in chunks of 32
 //   k_cull_place  the candidates in pair order: per block of words a scan, the block's
-//                 place by looking back over the earlier blocks' counts, one thread per candidate
+//                 place by looking back over the earlier blocks' counts (the decoupled look-back of
+//                 Merrill and Garland's single-pass scan, 2016), one thread per candidate
 // The all-pairs mode and the tuning's alternative make the bits in k_cull_place itself.
 //
 // 16,384 stacks (63 M pairs, 0.95 M candidates): the separate count, scan and write passes took 9 +

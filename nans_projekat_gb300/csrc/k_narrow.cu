@@ -1,11 +1,11 @@
 // Narrowphase: GJK per candidate pair, then EPA per hit.
 //
 //   k_gjk        one thread per pair, up to kGjkShort EvolveSimplex calls
-//   k_epa_tiny   one thread per hit, an 11-vertex / 16-face polytope (98 % of the EPAs)
+//   k_epa_tiny   one thread per hit, an 11-vertex / 16-face polytope (97 to 99 % of the EPAs)
 //   k_pair_warp  one warp per pair (nans_epa_warp.cuh, a 34-vertex / 64-face polytope in
 //                registers): the GJK runs that need more calls, the EPAs of hulls of many points
-//                and those the per-thread polytope does not hold; every pair of a step that has
-//                too few of them for a thread each
+//                (unless the step has very many pairs) and those the per-thread polytope does
+//                not hold; every pair of a step that has too few of them for a thread each
 //   k_gjk_long   the long GJK runs with a thread each, where there are very many
 //   k_epa_medium one warp per EPA beyond that, a 256-face polytope in shared memory with the
 //                reference's list semantics in full (tiers 3 and 4 are in k_epa_large.cu)
@@ -30,8 +30,8 @@
 // iteration would repeat it up to the cap.
 //
 // 16,384 stacks (0.95 M pairs a step): the per-thread EPA takes 275 us where the form with the
-// horizon inside the face loop and a 20-face polytope took 535, and 1 in 1,000 of the EPAs it sends
-// on goes beyond the pair tier (1 in 250 went to the 256-face tier before).
+// horizon inside the face loop and a 20-face polytope took 535, and at most 1 EPA in 2,000 goes beyond
+// the pair tier (steps 6 to 48).
 #include <algorithm>
 
 #include "nans_epa_warp.cuh"
@@ -584,7 +584,7 @@ __device__ __forceinline__ void handover_put(const DevWorld &w, const EpaFast &E
 // warp touches 32 consecutive words); the face list is an ordered list of slots in 4-bit steps of
 // one 64-bit word, so that removing faces moves nothing, and the horizon one byte per edge in
 // another. The support points SupA/SupB, read only for the final contact point, live in
-// thread-local arrays. 16 faces and 11 vertices (7 iterations) hold ~99% of the stack workload's
+// thread-local arrays. 16 faces and 11 vertices (7 iterations) hold 97 to 99 % of the stack workload's
 // EPAs.
 // ------------------------------------------------------------------------------------
 constexpr int kTinyThreads = 64;

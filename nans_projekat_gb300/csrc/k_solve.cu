@@ -8,9 +8,9 @@
 // number wave = 1 + max(last wave of body A, last wave of body B); contacts of one wave run
 // in parallel and waves run in order, which reproduces the sequential result bit for bit.
 //
-// Per scene: (1) compact the scene's hits in candidate order and (2) label their waves (one
-// thread, shared memory; a scene whose candidates fit one chunk keeps its hits in shared memory
-// throughout), (3) counting-sort the contacts by wave (wave sizes counted in shared memory),
+// Per scene: (1) compact the scene's hits in candidate order and (2) label their waves (a chunk of
+// many by all threads in rounds, what is left and short ones by one thread, in shared memory; a scene
+// whose candidates fit one chunk keeps its hits there throughout), (3) counting-sort the contacts by wave (wave sizes counted in shared memory),
 // (4) place each contact at its slot in wave order with everything that does not depend on
 // velocities (normal, tangents, lever arms, effective masses, the Baumgarte term), (5) per
 // wave, on a shared-memory copy of the scene's velocities: the 'iterations'-step

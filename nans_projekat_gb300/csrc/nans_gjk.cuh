@@ -18,7 +18,7 @@ __device__ __forceinline__ v3 triple_cross(v3 a, v3 b, v3 c) { return (dot3(c, a
 
 // len3(dir) <= 1e-4f (code/nans.cpp:748) without the square root: its correctly rounded value is at
 // most 1e-4f exactly when the squared length is at most kShortDir2, the largest float whose root is
-// (tests/test_gjk_paths.py checks the floats around it).
+// (tests/test_narrow_paths.py checks the floats around it).
 constexpr float kShortDir2 = 0x1.5798eep-27f;
 __device__ __forceinline__ bool dir_too_short(v3 d) { return dot3(d, d) <= kShortDir2; }
 

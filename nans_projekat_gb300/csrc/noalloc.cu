@@ -257,8 +257,7 @@ __device__ __forceinline__ void solve_one(const Floor &F, const float4 (&q)[9], 
 //   (1) the contacts' bodies, and per body how many contacts touch it;
 //   (2) each body's contacts side by side (a counting sort by body, order within a body free);
 //   (3) per contact and side, its neighbours in list order among its body's contacts, by looking
-//       through them (a few; a body that all 16,384 contacts touch costs one look at each per contact),
-//       and the velocity-independent constants;
+//       through them (a few, at most kOneLaunch), and the velocity-independent constants;
 //   (4) the waves, on a shared-memory copy of the velocities where they fit.
 // Bound by the waves' chain: a barrier, the constants' load (L2) and the impulses each. The form before
 // labelled the waves by one thread from global memory and ran the loop's friction bound in double
