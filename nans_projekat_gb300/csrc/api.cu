@@ -576,10 +576,11 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     // 0.410 ms a step at 122,000 bodies, 0.223 against 0.208 at 34,000. Hulls of many points always
     // take a warp (0.351 against 0.522 ms at 53,000 bodies).
     w->long_gjk = ndyn >= 80000 && !large_hulls;
-    // The first GJK pass's form for spheres (k_gjk) from a quarter of the bodies on, half where hulls of many
-    // points, which it leaves out, are among the others (301 to 4,096 mixed scenes of a quarter spheres
-    // and a third hulls: 0.3 to 0.8 % slower with it).
-    w->sphere_gjk = ts > 0 && 4 * ts >= (large_hulls ? 2 : 1) * (long long)ndyn;
+    // The first GJK pass's form for spheres (k_gjk) where they are half of the bodies (its gains are at k_gjk).
+    // With a quarter of them the lanes that wait cost as much as the pair tier saves: 300 scenes of 60
+    // boxes and 40 spheres 110 against 111 us a step, 4,096 mixed scenes 682 against 686 (three boxes and a
+    // sphere, 50,000 times, would gain: 661 against 599).
+    w->sphere_gjk = ts > 0 && 2 * ts >= (long long)ndyn;
     d.gjk_warp = (w->flags & NANS_WORLD_GJK_WARP) ? 1 : 0;
     d.sm_count = w->sm_count;
     d.giant_blocks = std::min(giant_grid(w->sm_count), upto(1, INT32_MAX) < 4096 ? 16 : INT32_MAX);

@@ -953,9 +953,9 @@ constexpr int kGjkShort = 8;
 // such a pair that is still evolving after kGjkShort calls, they go on to kGjkSphere calls in place
 // instead of taking a warp each on the pair tier. Hulls of many points and boxes do not: their runs are
 // longer. In worlds of many spheres (launch_gjk): 2,000 scenes of 20 spheres on the ground 291 -> 127 us a
-// step, 300 of them 114 -> 102, 100,000 scenes of a box and a sphere 787 -> 679, 50,000 of three boxes and
-// a sphere 661 -> 599. With one sphere among 32 boxes the lanes that wait cost more (1,000 such scenes
-// 169 -> 175), and the code alone 0.3 % of a step of 16,384 stacks, so those keep the plain form.
+// step, 300 of them 114 -> 102, 100,000 scenes of a box and a sphere 787 -> 679. With one sphere among 32
+// boxes the lanes that wait cost more (1,000 such scenes 169 -> 175), and the code alone 0.3 % of a step of
+// 16,384 stacks, so those keep the plain form.
 constexpr int kGjkSphere = 12, kGjkTogether = 4;
 
 struct SphereCalls

@@ -1,6 +1,6 @@
 """Worlds of many spheres against the oracle, bit for bit: the first GJK pass lets pairs with a sphere run on
-where a warp holds several of them. From a quarter of the bodies, half where hulls of more than eight
-points are among the others; steps of more than 2,432 candidates (below, every pair has a warp)."""
+where a warp holds several of them. From half of the bodies on, hulls of more than eight points among the
+others; steps of more than 2,432 candidates (below, every pair has a warp)."""
 import numpy as np
 import pytest
 
@@ -22,7 +22,7 @@ def _with_spheres(sc, n, seed, radius):
 
 
 @pytest.mark.parametrize("kind,n_scenes,boxes,spheres", [
-    ("stack", 1, 2, 8), ("stack", 180, 1, 20), ("stack", 1500, 1, 1), ("stack", 500, 6, 2), ("stack", 260, 12, 4),
+    ("stack", 1, 2, 8), ("stack", 180, 1, 20), ("stack", 1500, 1, 1), ("stack", 300, 6, 6), ("stack", 300, 7, 6),
     ("hulls", 200, 14, 16), ("hulls", 160, 14, 40)])
 def test_many_spheres(oracle_lib, kind, n_scenes, boxes, spheres):
     from nans_projekat_gb300 import scenes
