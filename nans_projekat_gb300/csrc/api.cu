@@ -658,7 +658,7 @@ int upload_impl(nans_world *w, uint32_t nscenes, const uint32_t *snc, const uint
     // the attribute is per device and per kernel, shared by every world on the device: set it to
     // the largest table any world may use, so that one world never lowers another's limit
     if (nans::solve_smem(max_bodies, d.solve_cache) > 48 * 1024)
-        CK((cudaError_t)solve_kernel_attrs(d, (int)kSolveSmemMax));
+        CK((cudaError_t)solve_kernel_attrs((int)kSolveSmemMax));
     CK(cudaStreamSynchronize(st));
     w->uploaded = true;
     w->graph_steps_run = 0;

@@ -1500,7 +1500,7 @@ __global__ void __launch_bounds__(kSceneThreads) k_scene_step(DevWorld w, float 
     __syncthreads(); // the warps' polytopes' memory becomes the solver's
     // (4) the solve, unless a pair of the scene went to the large tiers (the late pass)
     if (!s_late)
-        solve_scene<false>(w, s, dt, s_dyn, sh, s_maxw);
+        solve_scene<false, false>(w, s, dt, s_dyn, sh, s_maxw);
     // In a graph, the last block to finish opens the conditional node of the large tiers and the
     // late pass when a scene went late (work counter 13, counted by escalate); one call per launch.
     if (signal && tid == 0)

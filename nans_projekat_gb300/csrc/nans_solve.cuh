@@ -379,7 +379,7 @@ __device__ __forceinline__ void label_chunk(const DevWorld &w, int cb, int b0, i
 // sort by wave, (4) the placement with the velocity-independent constants, (5) the waves.
 // s_dyn is the dynamic shared memory solve_smem sizes, sh 32 ints and s_maxw one int of shared
 // memory. The caller synchronises the block before it reuses that memory.
-template <bool WARM>
+template <bool WARM, bool ORDERED>
 __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, float4 *s_dyn, int *sh, int &s_maxw)
 {
     int *const s_c = reinterpret_cast<int *>(s_dyn), *const s_ab = s_c + kWaveChunk, *const s_wv = s_ab + kWaveChunk,
@@ -531,10 +531,10 @@ __device__ __forceinline__ void solve_scene(const DevWorld &w, int s, float dt, 
     // scene of one chunk takes its hits from shared memory, a larger one from s_order.
     //
     // On a tape the order matters to rounding: the adjoint sums the gradients of restitution and friction
-    // over the slots. There a wave's contacts keep list order, so that the same rollout gives the same
+    // over the slots. There (ORDERED) a wave's contacts keep list order, so that the same rollout gives the same
     // gradients: one warp turns the waves into places 32 hits at a time (the atomics alone give the order of
     // a block's warps; a block of one warp has but one).
-    const bool ordered = !WARM && w.s_fwd != nullptr && blockDim.x > 32;
+    const bool ordered = ORDERED && blockDim.x > 32;
     if (ordered)
     {
         for (int base = 0; tid < 32 && base < nh; base += 32)
